@@ -25,6 +25,7 @@
 #include "host_pool.h"
 #include "kernels.cuh"
 #include "mlp.cuh"
+#include "pair.cuh"
 #include "tc_gemm.cuh"
 
 namespace {
@@ -89,6 +90,7 @@ struct HostGeom {
     // with q): host loops over the reference's grids walk them in memory
     // order instead of one column (stride nh*n) at a time
     std::vector<int> pt_ord;
+    int span = 0;           // lines that can be nonzero on either side of k = 0: kx < span, |ky| < span
     std::vector<int> yrun;  // 3 per line kx < KX (see Geom::yrun), empty if some line is not two runs
     std::vector<double> w;
 };
@@ -127,6 +129,8 @@ HostGeom build_geom(int n, const int *masker1, bool full)
         }
     h.ncol = (int)h.col_i.size();
     h.npw = (int)h.pt_k.size();
+    h.span = h.KX;
+    for (int j : h.col_j) h.span = std::max(h.span, j <= n / 2 ? j + 1 : n - j);
     h.pt_ord.reserve(h.npw);
     for (long idx = 0; idx < nfft3d; ++idx)
         if (h.inv_idx[idx] >= 0) h.pt_ord.push_back(h.inv_idx[idx]);
@@ -202,7 +206,8 @@ cudaError_t upload(DevArena &ar, X **d, const std::vector<X> &h)
 struct FftOps {
     virtual ~FftOps() = default;
     virtual size_t elem() const = 0;
-    virtual int init(DevArena &ar, int KX, int ncol) = 0;
+    // span: see HostGeom::span
+    virtual int init(DevArena &ar, int KX, int ncol, int span) = 0;
     virtual void inv_z(const Geom &g, const cx<double> *psi, long ldp, void *Tb, int nb, cudaStream_t s) = 0;
     virtual void fwd_z_store(const Geom &g, const void *Tb, cx<double> *out, long ldo, double scale,
                              int nb, cudaStream_t s) = 0;
@@ -210,9 +215,11 @@ struct FftOps {
     virtual void plane(int mode, const Geom &g, void *Tb, const PlaneArgs &a, int nchunks, cudaStream_t s) = 0;
     virtual int plane_ctas_per_sm(int mode) const = 0;  // resident CTAs of a plane pass
     virtual int plane_ctas_per_plane(int mode) const = 0;  // CTAs sharing one z plane (row split)
+    virtual int plane_bands(int mode) const = 0;           // bands a band pass transforms together
     // occupancy builds of a plane pass (1 or 2) and the one that runs
     virtual int plane_variants(int mode) const = 0;
     virtual int plane_variant(int mode) const = 0;
+    virtual int plane_builds(int mode) const = 0;  // how many of the choices run different builds
     virtual void set_plane_variant(int mode, int v) = 0;
 };
 
@@ -225,6 +232,22 @@ struct FftOpsT final : FftOps {
     size_t psmem_split = 0;  // the row-split density build (no staged columns)
     bool hi_fits[4] = {false, false, false, false};  // the high-occupancy build's CTAs fit an SM
     int occ[4] = {0, 0, 0, 0};                       // plane build that runs, per mode
+
+    // The band passes (density, V psi) take two bands as one complex field
+    // (pair.cuh).  One band a CTA (plane_kernel) is left for FP64 at n = 128
+    // where a sphere's lines of two bands do not fit shared memory (KX > 33).
+    static constexpr bool kOneBand = NF == 128 && sizeof(T) == 8;
+    // values per line end that can be nonzero in the pruned build (0: none
+    // built): half of a lane's inputs at n = 64, 6 of 16 at n = 128
+    static constexpr int kKZ = NF == 128 ? 3 : (NF == 64 ? 2 : 0);
+    struct Pair {
+        bool ok = false;      // the pass runs in pairs
+        size_t sm = 0;        // shared memory, without and with the staged columns (0: they do not fit)
+        size_t sm_stage = 0;
+        int per_sm = 1;       // resident CTAs
+    } pair[2];                // PM_DENSITY, PM_APPLYV
+    bool pruned = false;             // the sphere's lines fit the pruned build
+    const cx<T> *ptw = nullptr;      // PairTw tables
 
     size_t elem() const override { return sizeof(cx<T>); }
 
@@ -255,7 +278,65 @@ struct FftOpsT final : FftOps {
             for (int q = 0; q < L::Q; ++q) v[at + t * L::Q + q] = turn(q * t, N, sign);
     }
 
-    int init(DevArena &ar, int kx, int ncol) override
+    // the pair passes' forward table: W_N^-(t U + u) t' at (t' U + u) P + t
+    template <int N>
+    static void fill_pair_dif(std::vector<cx<T>> &v, int at)
+    {
+        using L = Line<N>;
+        for (int tp = 0; tp < L::P; ++tp)
+            for (int u = 0; u < L::U; ++u)
+                for (int t = 0; t < L::P; ++t) v[at + (tp * L::U + u) * L::P + t] = turn((t * L::U + u) * tp, N, -1);
+    }
+
+    // f(kernel) for a pair pass, pruned or not
+    template <int MODE, typename F>
+    auto with_pair(F &&f)
+    {
+        if constexpr (kKZ > 0)
+            if (pruned) return f(pair_kernel<T, NF, MODE, kKZ>);
+        return f(pair_kernel<T, NF, MODE, Line<NF>::Q / 2>);
+    }
+
+    template <int MODE>
+    int init_pair(int ncol, int optin)
+    {
+        Pair &p = pair[MODE];
+        p.sm = pair_smem_bytes<T, NF, MODE>(KX, ncol, false);
+        p.sm_stage = pair_smem_bytes<T, NF, MODE>(KX, ncol, true);
+        if ((int)p.sm_stage > optin) p.sm_stage = 0;  // the columns are read where they are used
+        if ((int)p.sm > optin) return CPSD_OK;
+        cudaError_t e = with_pair<MODE>([&](auto *k) { return allow_max_smem(k, optin); });
+        CK(e);
+        const size_t sm = p.sm_stage ? p.sm_stage : p.sm;
+        e = with_pair<MODE>([&](auto *k) {
+            return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p.per_sm, k, PairCfg<T, NF, MODE>::NT, sm);
+        });
+        CK(e);
+        p.per_sm = std::max(p.per_sm, 1);
+        p.ok = true;
+        // one build: either occupancy choice runs it
+        hi_fits[MODE] = true;
+        occ[MODE] = 1;
+        return CPSD_OK;
+    }
+
+    template <int MODE>
+    void bands(const Geom &g, void *Tb, const PlaneArgs &a, int nchunks, cudaStream_t s)
+    {
+        PairArgs pa{};
+        pa.chunk_b0 = a.chunk_b0;
+        pa.rho_part = a.rho_part;
+        pa.V = a.V;
+        pa.ne0 = a.ne0;
+        // a chunk of one pair has no next pair to copy ahead
+        pa.stage = a.chunk_bands > 2 && pair[MODE].sm_stage != 0;
+        const size_t sm = pa.stage ? pair[MODE].sm_stage : pair[MODE].sm;
+        with_pair<MODE>([&](auto *k) {
+            k<<<dim3(NF, (unsigned)nchunks), PairCfg<T, NF, MODE>::NT, sm, s>>>(g, (cx<T> *)Tb, pa, ptw);
+        });
+    }
+
+    int init(DevArena &ar, int kx, int ncol, int span) override
     {
         KX = kx;
         constexpr int H = NF / 2;
@@ -271,6 +352,13 @@ struct FftOpsT final : FftOps {
         cx<T> *d = nullptr;
         CK(upload(ar, &d, tab));
         tw = Twiddles<T>::template at<NF>(d);
+        std::vector<cx<T>> pt(PairTw<NF>::total);
+        fill_line<NF>(pt, PairTw<NF>::inv, +1);
+        fill_pair_dif<NF>(pt, PairTw<NF>::dif);
+        cx<T> *pd = nullptr;
+        CK(upload(ar, &pd, pt));
+        ptw = pd;
+        pruned = kKZ > 0 && span <= kKZ * Line<NF>::P;
 
         zsmem = z_smem_bytes<T, NF>();
         int dev = 0, optin = 0;
@@ -286,8 +374,10 @@ struct FftOpsT final : FftOps {
         // The limit is a per-kernel (process-wide) attribute shared by every
         // context on the device: set it to the device maximum, launch with
         // what this sphere needs.
-        CK(allow_plane<PM_DENSITY>(optin));
-        CK(allow_plane<PM_APPLYV>(optin));
+        if constexpr (kOneBand) {
+            CK(allow_plane<PM_DENSITY>(optin));
+            CK(allow_plane<PM_APPLYV>(optin));
+        }
         CK(allow_plane<PM_INVREAL>(optin));
         CK(allow_plane<PM_FWDREAL>(optin));
         // the high-occupancy build needs its CTAs' shared memory (plus the
@@ -308,7 +398,9 @@ struct FftOpsT final : FftOps {
         // lines in two CTAs: measured slower than the whole-plane build, so
         // it is only a candidate of the tuner
         if (plane_row_split<NF, PM_DENSITY, 2>() > 1) occ[PM_DENSITY] = 0;
-        return CPSD_OK;
+        int rc = init_pair<PM_DENSITY>(ncol, optin);
+        if (!rc) rc = init_pair<PM_APPLYV>(ncol, optin);
+        return rc;
     }
 
     template <int MODE>
@@ -360,25 +452,34 @@ struct FftOpsT final : FftOps {
     }
     void plane(int mode, const Geom &g, void *Tb, const PlaneArgs &a, int nchunks, cudaStream_t s) override
     {
-        // a CTA takes plane_bands_per_cta chunks (one band each for V psi)
-        dim3 grid(NF, (unsigned)cdiv(nchunks, plane_bands_per_cta(NF, mode)));
-        PlaneArgs pa = a;
-        pa.nchunks = nchunks;
+        const dim3 grid(NF, (unsigned)nchunks);
         const int nt = plane_threads<T, NF>(mode);
         switch (mode) {
-        case PM_DENSITY: launch_plane<PM_DENSITY>(grid, nt, g, Tb, pa, s); break;
-        case PM_APPLYV: launch_plane<PM_APPLYV>(grid, nt, g, Tb, pa, s); break;
-        case PM_INVREAL: launch_plane<PM_INVREAL>(grid, nt, g, Tb, pa, s); break;
-        default: launch_plane<PM_FWDREAL>(grid, nt, g, Tb, pa, s); break;
+        case PM_DENSITY:
+            if (pair[PM_DENSITY].ok) return bands<PM_DENSITY>(g, Tb, a, nchunks, s);
+            if constexpr (kOneBand) launch_plane<PM_DENSITY>(grid, nt, g, Tb, a, s);
+            break;
+        case PM_APPLYV:
+            if (pair[PM_APPLYV].ok) return bands<PM_APPLYV>(g, Tb, a, nchunks, s);
+            if constexpr (kOneBand) launch_plane<PM_APPLYV>(grid, nt, g, Tb, a, s);
+            break;
+        case PM_INVREAL: launch_plane<PM_INVREAL>(grid, nt, g, Tb, a, s); break;
+        default: launch_plane<PM_FWDREAL>(grid, nt, g, Tb, a, s); break;
         }
     }
-    bool mode_ok(int mode) const { return psmem[mode] != 0; }
-    int plane_ctas_per_sm(int mode) const override { return occ[mode & 3] ? 2 : 1; }
+    int plane_bands(int mode) const override { return mode < 2 && pair[mode].ok ? 2 : 1; }
+    int plane_ctas_per_sm(int mode) const override
+    {
+        if (mode < 2 && pair[mode].ok) return pair[mode].per_sm;
+        return occ[mode & 3] ? 2 : 1;
+    }
     int plane_ctas_per_plane(int mode) const override
     {
+        if (mode < 2 && pair[mode].ok) return 1;
         return (mode == PM_DENSITY && occ[PM_DENSITY]) ? plane_row_split<NF, PM_DENSITY, 2>() : 1;
     }
     int plane_variants(int mode) const override { return hi_fits[mode & 3] ? 2 : 1; }
+    int plane_builds(int mode) const override { return mode < 2 && pair[mode].ok ? 1 : plane_variants(mode); }
     int plane_variant(int mode) const override { return occ[mode & 3]; }
     void set_plane_variant(int mode, int v) override
     {
@@ -508,6 +609,8 @@ struct cpsd_gpu_ctx {
     double *dn_part = nullptr;
     int *chunk_bp = nullptr;
     int nchunk_bp[2] = {0, 0};
+    int dens_bands = 0, dens_bands_bp = 0;  // bands of the largest density chunk
+    int nchunk_v = 0, v_bands = 0;          // V psi: chunks (both spins) and the largest, of the bands this context steps
     int lag_cluster = 8;  // CTAs per cluster of the Lagrange solver (16 where schedulable)
     int lag_lb = 0;       // its row-tile width
     // learned preconditioner (optional): shells, stats, features, outputs
@@ -551,7 +654,7 @@ struct cpsd_gpu_ctx {
     cx<double> *ex1 = nullptr, *ex2 = nullptr, *ex3 = nullptr;
     double *beta = nullptr, *coefT = nullptr, *Mov = nullptr, *gws = nullptr, *lag = nullptr;
     double *lmd = nullptr, *hml = nullptr, *Edev = nullptr, *red = nullptr;
-    int *chunk_dens = nullptr, *chunk_band = nullptr, *flags = nullptr;
+    int *chunk_dens = nullptr, *chunk_v = nullptr, *flags = nullptr;
     // epilogue (allocated on first use): Jacobi workspace, eigenpairs, overlaps
     double *eigA = nullptr, *eigV = nullptr, *eigD = nullptr, *eigVec = nullptr, *ortho = nullptr;
     int *eig_sweeps = nullptr;
@@ -574,14 +677,62 @@ struct cpsd_gpu_ctx {
 
 namespace {
 
-// Band ranges of the density pass: n0 chunks of spin 0's ne0 bands, then
-// n1 chunks of spin 1's (starts, ends appended: n0 + n1 + 1 entries).
-std::vector<int> density_chunk_table(int ne0, int n0, int ne1, int n1)
+// Band ranges of a band pass (density, V psi): n0 chunks of spin 0's ne0
+// bands, then n1 chunks of spin 1's (starts, ends appended: n0 + n1 + 1
+// entries).  The passes take `unit` bands together: the chunks start on
+// multiples of it where there are enough such starts.
+std::vector<int> chunk_table(int ne0, int n0, int ne1, int n1, int unit)
 {
-    std::vector<int> b0;
-    for (int q = 0; q <= n0; ++q) b0.push_back((int)((long)ne0 * q / n0));
-    for (int q = 1; q <= n1; ++q) b0.push_back(ne0 + (int)((long)ne1 * q / n1));
+    std::vector<int> b0{0};
+    auto add = [&](int first, int ne, int nc) {
+        const long units = cdiv(ne, unit);
+        for (int q = 1; q <= nc; ++q)
+            b0.push_back(first + (nc <= units ? (int)std::min<long>(ne, unit * (units * q / nc)) : (int)((long)ne * q / nc)));
+    };
+    add(0, ne0, n0);
+    add(ne0, ne1, n1);
     return b0;
+}
+
+// The chunk count that minimises waves x (units of bands per CTA) over the
+// SMs' resident slots, the smallest such count (fewer partial densities, more
+// bands to copy ahead within a CTA).
+int best_chunks(int bands, int unit, int planes, long slots)
+{
+    const int units = (int)cdiv(bands, unit);
+    int best = 1;
+    long best_cost = -1;
+    for (int ch = 1; ch <= std::min(units, 64); ++ch) {
+        const long cost = cdiv((long)planes * ch, std::max<long>(slots, 1)) * cdiv(units, ch);
+        if (best_cost < 0 || cost < best_cost) {
+            best_cost = cost;
+            best = ch;
+        }
+    }
+    return best;
+}
+
+int largest_chunk(const std::vector<int> &tab, int nchunks)
+{
+    int m = 0;
+    for (int q = 0; q < nchunks; ++q) m = std::max(m, tab[q + 1] - tab[q]);
+    return m;
+}
+
+// The V psi pass's chunks of n0 bands of spin 0 and n1 of spin 1 (the bands
+// this context steps), for the build that runs now.
+int plan_v_chunks(cpsd_gpu_ctx *c, int n0, int n1)
+{
+    const int unit = c->fft->plane_bands(PM_APPLYV), halves = n0 > 0 && n1 > 0 ? 2 : 1;
+    const long slots = (long)c->sms * c->fft->plane_ctas_per_sm(PM_APPLYV);
+    const int ch0 = n0 > 0 ? best_chunks(n0, unit, halves * c->n, slots) : 0;
+    const int ch1 = n1 > 0 ? best_chunks(n1, unit, halves * c->n, slots) : 0;
+    const std::vector<int> tab = chunk_table(n0, ch0, n1, ch1, unit);
+    c->nchunk_v = ch0 + ch1;
+    c->v_bands = largest_chunk(tab, c->nchunk_v);
+    CK(cudaMemcpyAsync(c->chunk_v, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    return CPSD_OK;
 }
 
 // Split-K plan of a batch of weighted TN products: about two CTAs per SM
@@ -836,6 +987,8 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
         PlaneArgs pa{};
         pa.chunk_b0 = c->bp ? c->chunk_bp : c->chunk_dens;
         pa.rho_part = c->rho_part;
+        pa.chunk_bands = c->bp ? c->dens_bands_bp : c->dens_bands;
+        pa.ne0 = (c->ispin == 2) ? std::max(0, c->ne0 - lo) : nbl;
         const int ch0 = c->bp ? c->nchunk_bp[0] : c->nchunk0, ch1 = c->bp ? c->nchunk_bp[1] : c->nchunk1;
         if (ch0 + ch1 > 0) {
             c->fft->plane(PM_DENSITY, c->g, c->Tb, pa, ch0 + ch1, s);
@@ -928,10 +1081,11 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
         // (V + xc) psi back to G, -H psi and the SD step, cpsd.c:384-400
         if (nbl > 0) {
             PlaneArgs pp{};
-            pp.chunk_b0 = c->chunk_band;
+            pp.chunk_b0 = c->chunk_v;
+            pp.chunk_bands = c->v_bands;
             pp.V = c->Vr;
             pp.ne0 = (c->ispin == 2) ? std::max(0, c->ne0 - lo) : nbl;
-            c->fft->plane(PM_APPLYV, c->g, c->Tb, pp, nbl, s); c->nlaunch += 1;
+            c->fft->plane(PM_APPLYV, c->g, c->Tb, pp, c->nchunk_v, s); c->nlaunch += 1;
         }
         mark(c, 8);
         if (fork) CK(cudaStreamWaitEvent(s, c->ev_side, 0));  // kinetic + nonlocal c2 is in place
@@ -1256,7 +1410,7 @@ int cpsd_fft_run_full(int n, int dir, const Geom &g, double *grid, cx<double> *p
         CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
         c->inv_ok = (int)plane_need(n, PM_INVREAL, kx, 0) <= optin;
         c->fwd_ok = (int)plane_need(n, PM_FWDREAL, kx, 0) <= optin;
-        int rc = c->ops->init(c->ar, kx, 0);
+        int rc = c->ops->init(c->ar, kx, 0, n);
         if (rc) return rc;
         e = c.get();
         cache.push_back(std::move(c));
@@ -2007,11 +2161,11 @@ int cpsd_gpu_create(const cpsd_gpu_params *p, const int *masker1, cpsd_gpu_ctx *
     DevArena &ar = c->ar;
     c->fft64 = make_fft(c->n, CPSD_PREC_FP64);
     if (!c->fft64) return CPSD_ERR_GRID;
-    int rc = c->fft64->init(ar, h.KX, h.ncol);
+    int rc = c->fft64->init(ar, h.KX, h.ncol, h.span);
     if (rc) return rc;
     if (p->precision == CPSD_PREC_MIXED) {
         c->fft32 = make_fft(c->n, CPSD_PREC_MIXED);
-        rc = c->fft32->init(ar, h.KX, h.ncol);
+        rc = c->fft32->init(ar, h.KX, h.ncol, h.span);
         if (rc) return rc;
         CK(cudaFuncSetAttribute(tc_gemm_tn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
         CK(cudaFuncSetAttribute(tc_overlaps3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOvSmem));
@@ -2070,41 +2224,29 @@ int cpsd_gpu_create(const cpsd_gpu_params *p, const int *masker1, cpsd_gpu_ctx *
         CK(ar.alloc(&t, tbytes));
         c->Taux = t;
     }
-    // density chunks (bands summed by one CTA per z plane): the count that
-    // minimises waves x bands per CTA over the SMs' resident slots, the
-    // smallest such count (fewer partial densities to add); never across spins
+    // density chunks: bands summed by one CTA per z plane, never across spins
     {
         const long slots = (long)c->sms * c->fft->plane_ctas_per_sm(PM_DENSITY) /
                            c->fft->plane_ctas_per_plane(PM_DENSITY);
-        auto best_chunks = [&](int bands, int planes_per_chunk_group) {
-            int best = 1;
-            long best_cost = -1;
-            for (int ch = 1; ch <= std::min(bands, 64); ++ch) {
-                const long cost = cdiv((long)planes_per_chunk_group * ch, slots) * cdiv(bands, ch);
-                if (best_cost < 0 || cost < best_cost) {
-                    best_cost = cost;
-                    best = ch;
-                }
-            }
-            return best;
-        };
+        const int unit = c->fft->plane_bands(PM_DENSITY);
         if (c->ispin == 1) {
-            c->nchunk0 = best_chunks(c->ne0, c->n);
+            c->nchunk0 = best_chunks(c->ne0, unit, c->n, slots);
             c->nchunk1 = 0;
         } else {  // both spins share the launch: plan each with half of the slots
-            c->nchunk0 = best_chunks(c->ne0, 2 * c->n);
-            c->nchunk1 = c->ne1 > 0 ? best_chunks(c->ne1, 2 * c->n) : 0;
+            c->nchunk0 = best_chunks(c->ne0, unit, 2 * c->n, slots);
+            c->nchunk1 = c->ne1 > 0 ? best_chunks(c->ne1, unit, 2 * c->n, slots) : 0;
         }
         c->dens_model[0] = c->nchunk0;
         c->dens_model[1] = c->nchunk1;
         // room for up to max(4, 2 x the model's count) chunks per spin (tuning)
         c->dens_cap = std::min(std::max(4, 2 * std::max(c->nchunk0, c->nchunk1)), std::max(c->ne0, c->ne1));
-        std::vector<int> b0 = density_chunk_table(c->ne0, c->nchunk0, c->ne1, c->nchunk1);
+        std::vector<int> b0 = chunk_table(c->ne0, c->nchunk0, c->ne1, c->nchunk1, unit);
+        c->dens_bands = largest_chunk(b0, c->nchunk0 + c->nchunk1);
         b0.resize((size_t)2 * c->dens_cap + 1, 0);
         CK(upload(ar, &c->chunk_dens, b0));
-        std::vector<int> bb(nb + 1);
-        for (int b = 0; b <= nb; ++b) bb[b] = b;
-        CK(upload(ar, &c->chunk_band, bb));
+        CK(ar.alloc(&c->chunk_v, (size_t)nb + 1));
+        rc = plan_v_chunks(c.get(), c->ne0, c->ne1);
+        if (rc) return rc;
     }
     CK(ar.alloc(&c->rho_part, (size_t)(std::min(c->dens_cap, c->ne0) + std::min(c->dens_cap, c->ne1)) * c->n3));
     CK(ar.alloc(&c->dn, (size_t)c->ispin * c->n3));
@@ -2914,9 +3056,10 @@ int cpsd_gpu_set_band_range(cpsd_gpu_ctx *c, int lo, int hi)
 {
     if (!c) return CPSD_ERR_ARG;
     if (hi < 0) {  // back to stepping every band
+        CK(cudaSetDevice(c->prm.device));
         c->bp = false;
         drop_graphs(c);
-        return CPSD_OK;
+        return plan_v_chunks(c, c->ne0, c->ne1);
     }
     if (lo < 0 || lo > hi || hi > c->nb || c->mlp || c->move) return CPSD_ERR_ARG;
     CK(cudaSetDevice(c->prm.device));
@@ -2929,12 +3072,12 @@ int cpsd_gpu_set_band_range(cpsd_gpu_ctx *c, int lo, int hi)
     const int n0 = std::max(0, std::min(hi, c->ne0) - lo), n1 = (hi - lo) - n0;
     const int ch0 = n0 > 0 ? std::min(std::max(c->nchunk0, 1), n0) : 0;
     const int ch1 = n1 > 0 ? std::min(std::max(c->nchunk1, 1), n1) : 0;
-    std::vector<int> tab;
-    tab.push_back(0);
-    for (int q = 1; q <= ch0; ++q) tab.push_back((int)((long)n0 * q / ch0));
-    for (int q = 1; q <= ch1; ++q) tab.push_back(n0 + (int)((long)n1 * q / ch1));
+    const std::vector<int> tab = chunk_table(n0, ch0, n1, ch1, c->fft->plane_bands(PM_DENSITY));
+    c->dens_bands_bp = largest_chunk(tab, ch0 + ch1);
     CK(cudaMemcpyAsync(c->chunk_bp, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice, c->st));
     CK(cudaStreamSynchronize(c->st));
+    int rc = plan_v_chunks(c, n0, n1);
+    if (rc) return rc;
     c->nchunk_bp[0] = ch0;
     c->nchunk_bp[1] = ch1;
     c->bp_lo = lo;
@@ -3022,13 +3165,20 @@ int cpsd_gpu_set_tuning(cpsd_gpu_ctx *c, const cpsd_gpu_tuning *t)
     const int n0 = t->density_chunks;
     const int n1 = c->ispin == 2 && c->ne1 > 0 ? std::min(t->density_chunks, c->ne1) : 0;
     if (n0 != c->nchunk0 || n1 != c->nchunk1) {
-        const std::vector<int> tab = density_chunk_table(c->ne0, n0, c->ne1, n1);
+        const std::vector<int> tab = chunk_table(c->ne0, n0, c->ne1, n1, c->fft->plane_bands(PM_DENSITY));
+        c->dens_bands = largest_chunk(tab, n0 + n1);
         CK(cudaMemcpyAsync(c->chunk_dens, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice, c->st));
         CK(cudaStreamSynchronize(c->st));
         c->nchunk0 = n0;
         c->nchunk1 = n1;
     }
     for (int m = 0; m < 4; ++m) c->fft->set_plane_variant(m, t->plane_occupancy[m]);
+    {  // the V psi build sets how many CTAs are resident
+        const int lo = c->bp ? c->bp_lo : 0, hi = c->bp ? c->bp_hi : c->nb;
+        const int b0 = std::max(0, std::min(hi, c->ne0) - lo);
+        const int rc = plan_v_chunks(c, b0, (hi - lo) - b0);
+        if (rc) return rc;
+    }
     c->tn_ctas = t->tn_ctas_per_sm;
     if (!small) c->lag_tile = t->lagrange_solver == 1;
     drop_graphs(c);  // the step graphs hold the old choices
@@ -3155,7 +3305,7 @@ int cpsd_gpu_autotune(cpsd_gpu_ctx *c, int steps, int force, float *ms_before, f
         return cpsd_gpu_set_tuning(c, &cur);
     };
     for (int m = 0; m < 4 && !rc; ++m)
-        for (int v = 0; v <= lim.plane_occupancy[m] && !rc; ++v) rc = try_value(&cur.plane_occupancy[m], v);
+        for (int v = c->fft->plane_builds(m) > 1 ? 0 : lim.plane_occupancy[m] + 1; v <= lim.plane_occupancy[m] && !rc; ++v) rc = try_value(&cur.plane_occupancy[m], v);
     {
         const int model = c->dens_model[0];
         const int cand[4] = {1, std::max(1, model / 2), model + 1, 2 * model};
