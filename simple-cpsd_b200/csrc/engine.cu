@@ -26,6 +26,7 @@
 #include "kernels.cuh"
 #include "mlp.cuh"
 #include "pair.cuh"
+#include "small.cuh"
 #include "tc_gemm.cuh"
 
 namespace {
@@ -594,6 +595,7 @@ struct cpsd_gpu_ctx {
     cudaEvent_t ev_dn = nullptr;
     bool rec_dn = false;
     cudaStream_t cs = nullptr;  // the stream the GEMM helpers launch on
+    unsigned *ticket = nullptr;  // CTAs of the running small_overlap_kernel that are done
     bool lag_tile = false;  // 4 x 4 tiled solver (<= 128 bands, 16-CTA clusters schedulable)
     bool lag_tile_ok = false;  // the tiled solver can run on this device for these bands
     // tuning (cpsd_gpu_set_tuning / cpsd_gpu_autotune): split-K target of the
@@ -865,6 +867,110 @@ const double *Mblk(cpsd_gpu_ctx *c, int ms, int which)
     return c->Mov + ((long)ms * 4 + which) * (long)c->ne0 * c->ne0;
 }
 
+// Cells of at most 32 bands per spin take the 8 x 8 tile kernels of small.cuh
+// for their band-by-band products, in every GEMM mode: at 16 bands (64^3) the
+// three overlaps and the solver take 7 us there against 29 us as 64 x 64 tiles
+// (FP64, or 3xTF32 on 128 x 128 ones), a reduction and a solver launch.
+bool small_cell(const cpsd_gpu_ctx *c) { return c->ne0 <= kLagSmallMax; }
+
+template <int MODE, int MT>
+int launch_small(cpsd_gpu_ctx *c, const SmallArgs &a)
+{
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kSmCluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)a.splits, (unsigned)c->ispin);
+    cfg.blockDim = dim3(kSmThreads);
+    cfg.dynamicSmemBytes = small_smem_bytes<MODE, MT>(c->ne0);
+    cfg.stream = c->cs;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CK(cudaLaunchKernelEx(&cfg, small_overlap_kernel<MODE, MT>, a));
+    c->nlaunch += 1;
+    return CPSD_OK;
+}
+
+// A'WB of every spin's bands (small.cuh), MODE SM_LAGRANGE with a.lag set
+template <int MODE>
+int small_overlaps(cpsd_gpu_ctx *c, SmallArgs a, const double *A, const double *B)
+{
+    a.K = 2 * c->npw_pad;
+    a.ld = 2L * c->npw_pad;
+    a.w = c->w;
+    a.part = c->gws;
+    a.ticket = c->ticket;
+    for (int ms = 0; ms < c->ispin; ++ms) {
+        a.m[ms] = ms ? c->ne1 : c->ne0;
+        a.A[ms] = A + (ms ? c->ne0 : 0) * a.ld;
+        a.B[ms] = B + (ms ? c->ne0 : 0) * a.ld;
+    }
+    // at least four k-steps of 8 reals per warp, at most a CTA per SM
+    a.splits = kSmCluster * (int)std::min<long>(kSmMaxClusters, std::max<long>(1, cdiv(a.K / 8, 4L * kSmWarps * kSmCluster)));
+    switch (cdiv(c->ne0, 8)) {
+    case 1: return launch_small<MODE, 1>(c, a);
+    case 2: return launch_small<MODE, 2>(c, a);
+    case 3: return launch_small<MODE, 3>(c, a);
+    default: return launch_small<MODE, 4>(c, a);
+    }
+}
+
+// C_ms[i][j] = <A_i|B_j> over the bands of each spin (Gamma-point weights)
+int band_products(cpsd_gpu_ctx *c, const double *A, const double *B, double *const *C, int which = 0)
+{
+    if (small_cell(c)) {
+        SmallArgs a{};
+        for (int ms = 0; ms < c->ispin; ++ms) a.C[ms] = C[ms];
+        return small_overlaps<SM_ONE>(c, a, A, B);
+    }
+    const long ldr = 2L * c->npw_pad;
+    for (int ms = 0; ms < c->ispin; ++ms) {
+        const int m = ms ? c->ne1 : c->ne0;
+        const long off = (long)(ms ? c->ne0 : 0) * ldr;
+        const int rc = gemm_tn(c, m, m, 2 * c->npw_pad, A + off, ldr, B + off, ldr, c->w, 1.0, 0.0, C[ms], m, which);
+        if (rc) return rc;
+    }
+    return CPSD_OK;
+}
+
+// Out_j = beta Out_j + alpha sum_l mat_ms[l + j m] In_l over the bands of each spin
+void band_rotation(cpsd_gpu_ctx *c, double alpha, const double *const *mat, const double *In, double beta, double *Out,
+                   int which = 0)
+{
+    const long ldr = 2L * c->npw_pad;
+    if (small_cell(c)) {
+        SmallNNArgs a{};
+        a.K = 2 * c->npw_pad;
+        a.ld = ldr;
+        a.alpha = alpha;
+        a.beta = beta;
+        for (int ms = 0; ms < c->ispin; ++ms) {
+            const long off = (long)(ms ? c->ne0 : 0) * ldr;
+            a.m[ms] = ms ? c->ne1 : c->ne0;
+            a.mat[ms] = mat[ms];
+            a.in[ms] = In + off;
+            a.out[ms] = Out + off;
+        }
+        // a warp per 16 reals of the rows, up to two CTAs per SM
+        const dim3 grid((unsigned)std::min<long>(2L * c->sms, cdiv(a.K / 16, kSmWarps)), (unsigned)c->ispin);
+        switch (cdiv(c->ne0, 8)) {
+        case 1: small_nn_kernel<1><<<grid, kSmThreads, 0, c->cs>>>(a); break;
+        case 2: small_nn_kernel<2><<<grid, kSmThreads, 0, c->cs>>>(a); break;
+        case 3: small_nn_kernel<3><<<grid, kSmThreads, 0, c->cs>>>(a); break;
+        default: small_nn_kernel<4><<<grid, kSmThreads, 0, c->cs>>>(a); break;
+        }
+        c->nlaunch += 1;
+        return;
+    }
+    for (int ms = 0; ms < c->ispin; ++ms) {
+        const int m = ms ? c->ne1 : c->ne0;
+        const long off = (long)(ms ? c->ne0 : 0) * ldr;
+        gemm_nn(c, m, 2 * c->npw_pad, m, alpha, mat[ms], m, In + off, ldr, beta, Out + off, ldr, which);
+    }
+}
+
 const char *const kPhaseNames[] = {
     "inv_z_bands", "density_plane", "density_xc", "rho_fft",     "vloc_proj",  "potential_fft",
     "kinetic_nonlocal", "applyv_plane", "fwd_z_sd", "overlaps", "lagrange", "constraint",
@@ -1111,17 +1217,11 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
             // The residual R = cpsi - C1 (C1' W cpsi) per spin: only R is
             // preconditioned, so the update is plain SD wherever R = 0 and the
             // fixed point H psi = psi Lambda is that of plain SD.
-            for (int ms = 0; ms < c->ispin; ++ms) {
-                const int m = ms ? c->ne1 : c->ne0;
-                const long off = (long)(ms ? c->ne0 : 0) * ldr;
-                double *Mt = c->pM + (long)ms * c->ne0 * c->ne0;  // Mt[b][a] = <cpsi_b|c1_a>
-                int rc = gemm_tn(c, m, m, K, (const double *)c->cpsi + off, ldr, (const double *)c1 + off, ldr, c->w,
-                                 1.0, 0.0, Mt, m, TN_PROJECTOR);
-                if (rc) return rc;
-                // pR = -C1 Mt; the update adds cpsi (R = cpsi + pR)
-                gemm_nn(c, m, K, m, -1.0, Mt, m, (const double *)c1 + off, ldr, 0.0, (double *)c->pR + off, ldr,
-                        TN_PROJECTOR);
-            }
+            double *Mt[2] = {c->pM, c->pM + (long)c->ne0 * c->ne0};  // Mt[b][a] = <cpsi_b|c1_a>
+            int rc = band_products(c, (const double *)c->cpsi, (const double *)c1, Mt, TN_PROJECTOR);
+            if (rc) return rc;
+            // pR = -C1 Mt; the update adds cpsi (R = cpsi + pR)
+            band_rotation(c, -1.0, Mt, (const double *)c1, 0.0, (double *)c->pR, TN_PROJECTOR);
             band_stats_kernel<<<c->nb, 256, 0, s>>>(c->npw, c->ldc, c->w, c->tg, c1, c->cpsi, c->pstats);
             prec_mlp_kernel<<<mlp_forward_blocks((long)c->nb * kShells), kMlpTileThreads, 0, s>>>(
                 c->nb, c->tmax, c->pstats, c->dstep, c->mlp->wq, c->mlp->p, c->py);
@@ -1140,6 +1240,22 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
     la.ne1 = c->ne1;
     la.dte = c->dte;
     const long ne02 = (long)c->ne0 * c->ne0;
+    la.lmd = c->lmd;
+    la.fail = c->flags;
+    const double *lmds[2] = {c->lmd, c->lmd + ne02};
+    if (small_cell(c)) {  // overlaps and solver in one launch
+        SmallArgs a{};
+        a.lag = la;
+        int rc = small_overlaps<SM_LAGRANGE>(c, a, (const double *)c2, (const double *)c1);
+        if (rc) return rc;
+        mark(c, 10);
+        mark(c, 11);
+        band_rotation(c, c->dte, lmds, (const double *)c1, 1.0, (double *)c2);
+        mark(c, 12);
+        CK(cudaGetLastError());
+        c->cur ^= 1;
+        return CPSD_OK;
+    }
     for (int ms = 0; ms < c->ispin; ++ms) {
         const int m = ms ? c->ne1 : c->ne0;
         const long off = (long)(ms ? c->ne0 : 0) * ldr;
@@ -1160,13 +1276,9 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
     la.st1 = c->lag + 4 * ne02;
     la.X0 = c->lag + 5 * ne02;
     la.X1 = c->lag + 6 * ne02;
-    la.lmd = c->lmd;
     la.red = c->red;
-    la.fail = c->flags;
     la.lb = c->lag_lb;
-    if (c->ne0 <= kLagSmallMax)
-        lagrange_small_kernel<<<1, kLagThreads, lag_small_smem_bytes(c->ne0), s>>>(la);
-    else if (c->lag_tile) {
+    if (c->lag_tile) {
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1198,12 +1310,7 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
     c->nlaunch += 1;
     mark(c, 11);
     // constraint correction c2 += dte C1 lmd, cpsd.c:482-488
-    for (int ms = 0; ms < c->ispin; ++ms) {
-        const int m = ms ? c->ne1 : c->ne0;
-        const long off = (long)(ms ? c->ne0 : 0) * ldr;
-        gemm_nn(c, m, K, m, c->dte, c->lmd + ms * ne02, m, (const double *)c1 + off, ldr, 1.0,
-                (double *)c2 + off, ldr, TN_OVERLAPS);
-    }
+    band_rotation(c, c->dte, lmds, (const double *)c1, 1.0, (double *)c2, TN_OVERLAPS);
     mark(c, 12);
     CK(cudaGetLastError());
     c->cur ^= 1;
@@ -1328,17 +1435,12 @@ int energies(cpsd_gpu_ctx *c, int inner)
 {
     cudaStream_t s = c->st;
     const cx<double> *c2 = c->cbuf[c->cur], *c1 = c->cbuf[c->cur ^ 1];
-    const int K = 2 * c->npw_pad;
-    const long ldr = 2L * c->npw_pad;
     FinalArgs fa{};
-    for (int ms = 0; ms < c->ispin; ++ms) {
-        const int m = ms ? c->ne1 : c->ne0;
-        const long off = (long)(ms ? c->ne0 : 0) * ldr;
-        int rc = gemm_tn(c, m, m, K, (const double *)c1 + off, ldr, (const double *)c->cpsi + off, ldr, c->w,
-                         1.0, 0.0, (double *)Mblk(c, ms, 3), m);
-        if (rc) return rc;
-        fa.Mh[ms] = Mblk(c, ms, 3);
-    }
+    double *Mh[2] = {(double *)Mblk(c, 0, 3), (double *)Mblk(c, 1, 3)};
+    int rc = band_products(c, (const double *)c1, (const double *)c->cpsi, Mh);
+    if (rc) return rc;
+    fa.Mh[0] = Mh[0];
+    fa.Mh[1] = Mh[1];
     packed_terms_kernel<<<c->pblocks, 256, 0, s>>>(c->npw, c->w, c->sfac, c->vg, c->dng, c->vc, c->vall,
                                                    c->ppart); c->nlaunch += 1;
     band_terms_kernel<<<dim3(c->bblocks, c->nb), 256, 0, s>>>(c->npw, c->ldc, c->w, c->tg, c1, c2, c->bpart); c->nlaunch += 1;
@@ -2269,6 +2371,7 @@ int cpsd_gpu_create(const cpsd_gpu_params *p, const int *masker1, cpsd_gpu_ctx *
     CK(ar.alloc(&c->red, 2 * kLagClusterMax));
     CK(ar.alloc(&c->Edev, 16));
     CK(ar.alloc(&c->flags, 4));
+    CK(ar.alloc(&c->ticket, 1));
     c->gemm_splits_cap = 512;
     // split-K partials: at least 32 MB, and room for one split per SM of the
     // three overlaps of the largest spin
@@ -2302,9 +2405,25 @@ int cpsd_gpu_create(const cpsd_gpu_params *p, const int *masker1, cpsd_gpu_ctx *
     CK(ar.alloc(&c->pM, (size_t)c->ispin * c->ne0 * c->ne0));
     CK(ar.alloc(&c->pstats, (size_t)3 * nb));
     CK(ar.alloc(&c->py, (size_t)nb * kShells));
-    if (c->ne0 <= kLagSmallMax)
-        CK(cudaFuncSetAttribute(lagrange_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)lag_small_smem_bytes(kLagSmallMax)));
+    if (small_cell(c.get())) {
+        auto allow = [&](auto one, auto lag, size_t so, size_t sl) {
+            cudaError_t e = cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)so);
+            return e != cudaSuccess ? e : cudaFuncSetAttribute(lag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sl);
+        };
+        cudaError_t e = cudaSuccess;
+        const int top = kLagSmallMax;  // the attribute is the kernel's, shared by every context
+        switch (cdiv(c->ne0, 8)) {
+        case 1: e = allow(small_overlap_kernel<SM_ONE, 1>, small_overlap_kernel<SM_LAGRANGE, 1>,
+                          small_smem_bytes<SM_ONE, 1>(top), small_smem_bytes<SM_LAGRANGE, 1>(top)); break;
+        case 2: e = allow(small_overlap_kernel<SM_ONE, 2>, small_overlap_kernel<SM_LAGRANGE, 2>,
+                          small_smem_bytes<SM_ONE, 2>(top), small_smem_bytes<SM_LAGRANGE, 2>(top)); break;
+        case 3: e = allow(small_overlap_kernel<SM_ONE, 3>, small_overlap_kernel<SM_LAGRANGE, 3>,
+                          small_smem_bytes<SM_ONE, 3>(top), small_smem_bytes<SM_LAGRANGE, 3>(top)); break;
+        default: e = allow(small_overlap_kernel<SM_ONE, 4>, small_overlap_kernel<SM_LAGRANGE, 4>,
+                           small_smem_bytes<SM_ONE, 4>(top), small_smem_bytes<SM_LAGRANGE, 4>(top)); break;
+        }
+        CK(e);
+    }
     else {
         // 16-CTA clusters where the device can schedule them, else the portable 8
         CK(cudaFuncSetAttribute(lagrange_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -2581,21 +2700,16 @@ int cpsd_gpu_epilogue(cpsd_gpu_ctx *c, double *ortho, double *eig, double *vec)
     }
     const cudaStream_t cs_saved = c->cs;
     c->cs = s;
-    const int K = 2 * c->npw_pad;
-    const long ldr = 2L * c->npw_pad;
     const double *c1 = (const double *)c->cbuf[c->cur ^ 1];
     const double *c2 = (const double *)c->cbuf[c->cur];
     // orthonormality of c1 (main.c:455-467): <c1_i|c1_j>, Gamma-point dots
     if (ortho) {
-        for (int ms = 0; ms < c->ispin; ++ms) {
-            const int m = ms ? c->ne1 : c->ne0;
-            const long off = (long)(ms ? c->ne0 : 0) * ldr;
-            // row-major M x M from the TN product equals its column-major transpose (symmetric)
-            const int rc = gemm_tn(c, m, m, K, c1 + off, ldr, c1 + off, ldr, c->w, 1.0, 0.0, c->ortho + ms * ne02, m);
-            if (rc) {
-                c->cs = cs_saved;
-                return rc;
-            }
+        // row-major M x M from the TN product equals its column-major transpose (symmetric)
+        double *const Co[2] = {c->ortho, c->ortho + ne02};
+        const int rc = band_products(c, c1, c1, Co);
+        if (rc) {
+            c->cs = cs_saved;
+            return rc;
         }
     }
     // eigenpairs of hml per spin (main.c:470-479)
@@ -2612,12 +2726,8 @@ int cpsd_gpu_epilogue(cpsd_gpu_ctx *c, double *ortho, double *eig, double *vec)
     jacobi_eig_kernel<<<c->ispin, kEigThreads, 0, s>>>(ea);
     c->nlaunch += 1;
     // c1 <- c2 V per spin (main.c:481-487): band j of c1 = sum_l V[l][j] band l of c2
-    double *c1w = (double *)c->cbuf[c->cur ^ 1];
-    for (int ms = 0; ms < c->ispin; ++ms) {
-        const int m = ms ? c->ne1 : c->ne0;
-        const long off = (long)(ms ? c->ne0 : 0) * ldr;
-        gemm_nn(c, m, K, m, 1.0, c->eigVec + ms * ne02, m, c2 + off, ldr, 0.0, c1w + off, ldr);
-    }
+    const double *const V[2] = {c->eigVec, c->eigVec + ne02};
+    band_rotation(c, 1.0, V, c2, 0.0, (double *)c->cbuf[c->cur ^ 1]);
     c->cs = cs_saved;
     CK(cudaGetLastError());
     int sweeps[2] = {0, 0};
