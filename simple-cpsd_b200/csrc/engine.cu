@@ -577,6 +577,7 @@ struct cpsd_gpu_ctx {
     // per (steps, parity); a few kept
     struct MultiGraph {
         int steps, par, launches;
+        bool first;  // starts with a call's first step
         cudaGraphExec_t exec;
     };
     std::vector<MultiGraph> mgraphs;
@@ -594,6 +595,7 @@ struct cpsd_gpu_ctx {
     // so that its copy to the host can start during the rest of the step
     cudaEvent_t ev_dn = nullptr;
     bool rec_dn = false;
+    bool with_sf = true;  // the step forms the structure factors and projectors
     cudaStream_t cs = nullptr;  // the stream the GEMM helpers launch on
     unsigned *ticket = nullptr;  // CTAs of the running small_overlap_kernel that are done
     bool lag_tile = false;  // 4 x 4 tiled solver (<= 128 bands, 16-CTA clusters schedulable)
@@ -791,6 +793,16 @@ int launch_tn(int M, int N, int K, int nprod, const double *const *A, long lda, 
 // the constraint correction c2 += dte C1 lmd.
 enum { TN_PROJECTOR = 1, TN_OVERLAPS = 2 };
 
+// Whether a product of M x N outputs per sum (or an M x N matrix times the
+// bands) runs on the tensor cores: its 128 x 128 tiles lose to the 64 x 64 FP64
+// ones while they are mostly padding (32 projectors x 16 bands: the projector
+// products of a step take 27 us on tcgen05 and 21 us in FP64; 256 x 128: 176
+// and 280 us).
+bool tc_product(const cpsd_gpu_ctx *c, int which, int M, int N)
+{
+    return (c->gemm_mode & which) != 0 && c->precision == CPSD_PREC_MIXED && (long)M * N > 64 * 64;
+}
+
 // Batched weighted TN products of a context; `which` names the product so
 // that the tensor-core variant runs where the context runs mixed precision
 // and its GEMM mode includes that product.
@@ -800,7 +812,7 @@ int gemm_tn_batch(cpsd_gpu_ctx *c, int M, int N, int K, int nprod, const double 
 {
     if (M <= 0 || N <= 0 || nprod <= 0) return CPSD_OK;
     if (nprod > kTnMaxProd) return CPSD_ERR_ARG;
-    const bool tc = (c->gemm_mode & which) != 0 && c->precision == CPSD_PREC_MIXED;
+    const bool tc = tc_product(c, which, M, N);
     c->nlaunch += launch_tn(M, N, K, nprod, A, lda, B, ldb, w, alpha, beta, C, ldc, tc, c->gws, c->gemm_ws_elems,
                             c->flags + 2, c->cs, c->tn_ctas);
     return CPSD_OK;
@@ -850,7 +862,7 @@ void gemm_nn(cpsd_gpu_ctx *c, int NJ, int K, int L, double alpha, const double *
              const double *B, long ldb, double beta, double *Out, long ldo, int which = 0)
 {
     if (NJ <= 0 || L <= 0) return;
-    if ((c->gemm_mode & which) != 0 && c->precision == CPSD_PREC_MIXED) {
+    if (tc_product(c, which, NJ, L)) {
         dim3 grid((unsigned)cdiv(K, kTcN), (unsigned)cdiv(NJ, kTcM));
         tc_gemm_nn_kernel<<<grid, kTcThreads, kTcSmem, c->cs>>>(NJ, K, L, alpha, Mat, ldm, B, ldb, beta, Out, ldo,
                                                                 c->flags + 2);
@@ -1051,6 +1063,13 @@ int issue_knl(cpsd_gpu_ctx *c, cudaStream_t side, const cx<double> *c1, cx<doubl
     return CPSD_OK;
 }
 
+// r1 <- r2 at the start of a step, cpsd.c:174
+cudaError_t copy_positions(cpsd_gpu_ctx *c, cudaStream_t s)
+{
+    if (c->nion == 0) return cudaSuccess;
+    return cudaMemcpyAsync(c->r1, c->r2, sizeof(double) * 3 * c->nion, cudaMemcpyDeviceToDevice, s);
+}
+
 // One SD step in three phases.  A context that steps every band runs them
 // back to back (one_step); a band-parallel context (c->bp) steps only its
 // bands [bp_lo, bp_hi) in phases 0 and 1, and its caller exchanges between
@@ -1071,16 +1090,29 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
     // With phase timing on, everything stays on one stream so the phases add up.
     const bool fork = !c->phase_timing;
     cudaStream_t side = fork ? c->st2 : s;
+    // With fixed ions the structure factors and projectors of a call's first
+    // step hold for all its steps (and r1 <- r2 happens once): with_sf is false
+    // for the later ones, which fork the projector products off after the
+    // density pass instead (beside the small transforms; at the start they
+    // would compete with it).  128^3 / 64 ions: 84 us a step of the side stream.
+    const bool with_sf = c->with_sf || c->move || c->bp;
     if (phase == 0) {
-        CK(cudaMemcpyAsync(c->r1, c->r2, sizeof(double) * 3 * c->nion, cudaMemcpyDeviceToDevice, s));  // cpsd.c:174
-        if (fork) {
+        if (with_sf) CK(copy_positions(c, s));
+        auto side_work = [&]() -> int {
             CK(cudaEventRecord(c->ev_fork, s));
             CK(cudaStreamWaitEvent(c->st2, c->ev_fork, 0));
-            issue_sf(c, side);
-            CK(cudaEventRecord(c->ev_sf, c->st2));
+            if (with_sf) {
+                issue_sf(c, side);
+                CK(cudaEventRecord(c->ev_sf, c->st2));
+            }
             int rc = issue_knl(c, side, c1, c2, lo, nbl);
             if (rc) return rc;
             CK(cudaEventRecord(c->ev_side, c->st2));
+            return CPSD_OK;
+        };
+        if (fork && with_sf) {
+            int rc = side_work();
+            if (rc) return rc;
         }
 
         mark(c, 0);
@@ -1099,6 +1131,10 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
         if (ch0 + ch1 > 0) {
             c->fft->plane(PM_DENSITY, c->g, c->Tb, pa, ch0 + ch1, s);
             c->nlaunch += 1;
+        }
+        if (fork && !with_sf) {
+            int rc = side_work();
+            if (rc) return rc;
         }
         mark(c, 2);
         XcArgs xa{c->n3, c->ispin, ch0, ch1, c->rho_part, c->scal1, c->scal2, c->dn, c->xcp, c->xce, c->rfwd};
@@ -1134,9 +1170,9 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
         c->fft->plane(PM_FWDREAL, c->g, c->Taux, pf, 1, s); c->nlaunch += 1;
         c->fft->fwd_z_store(c->g, c->Taux, c->dng, c->ldc, 1.0, 1, s); c->nlaunch += 1;
         mark(c, 4);
-        if (fork)
+        if (fork && with_sf)
             CK(cudaStreamWaitEvent(s, c->ev_sf, 0));
-        else
+        else if (!fork)
             issue_sf(c, side);
         // V(G), cpsd.c:373-379
         vg_kernel<<<(unsigned)cdiv(c->npw, 128), 128, 0, s>>>(c->npw, c->vall, c->dng, c->vc, c->scal2, c->Vg);
@@ -1375,6 +1411,7 @@ constexpr size_t kMultiGraphs = 4;
 
 int run_steps(cpsd_gpu_ctx *c, int inner)
 {
+    bool first = true;
     if (!c->use_graph || c->phase_timing) {
         c->rec_dn = true;
         for (int it = 0; it < inner; ++it) {
@@ -1392,7 +1429,7 @@ int run_steps(cpsd_gpu_ctx *c, int inner)
         const int par = c->cur;
         cpsd_gpu_ctx::MultiGraph *m = nullptr;
         for (auto &x : c->mgraphs)
-            if (x.steps == k && x.par == par) m = &x;
+            if (x.steps == k && x.par == par && x.first == first) m = &x;
         if (!m) {
             cudaGraph_t g = nullptr;
             const long long before = c->nlaunch;
@@ -1400,9 +1437,11 @@ int run_steps(cpsd_gpu_ctx *c, int inner)
             int rc = CPSD_OK;
             for (int it = 0; it < k && !rc; ++it) {
                 c->rec_dn = it == k - 1;  // one record of ev_dn per graph, in its last step
+                c->with_sf = first && it == 0;
                 rc = one_step(c);
             }
             c->rec_dn = false;
+            c->with_sf = true;
             cudaError_t e = cudaStreamEndCapture(c->st, &g);
             c->cur = par;  // capture launched nothing: undo the buffer flips
             const int launches = (int)(c->nlaunch - before);
@@ -1420,12 +1459,13 @@ int run_steps(cpsd_gpu_ctx *c, int inner)
                 cudaGraphExecDestroy(c->mgraphs.front().exec);
                 c->mgraphs.erase(c->mgraphs.begin());
             }
-            c->mgraphs.push_back({k, par, launches, ex});
+            c->mgraphs.push_back({k, par, launches, first, ex});
             m = &c->mgraphs.back();
         }
         CK(cudaGraphLaunch(m->exec, c->st));
         c->nlaunch += m->launches;
         if (k & 1) c->cur ^= 1;
+        first = false;
         inner -= k;
     }
     return CPSD_OK;
@@ -1545,8 +1585,10 @@ struct cpsd_gpu_batch {
     std::vector<cpsd_gpu_ctx *> cells;
     cudaStream_t st = nullptr;
     std::vector<cudaEvent_t> ev;  // fork + one join per cell
-    cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-    int graph_launches = 0;
+    // one SD step of every cell, per parity of the orbital buffers; [1]: a
+    // call's first step (with the structure factors and projectors)
+    cudaGraphExec_t gexec[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+    int graph_launches[2] = {0, 0};
     long long nlaunch = 0;
 };
 
@@ -1554,17 +1596,19 @@ namespace {
 
 void batch_drop_graphs(cpsd_gpu_batch *b)
 {
-    for (auto &g : b->gexec)
-        if (g) {
-            cudaGraphExecDestroy(g);
-            g = nullptr;
-        }
+    for (auto &f : b->gexec)
+        for (auto &g : f)
+            if (g) {
+                cudaGraphExecDestroy(g);
+                g = nullptr;
+            }
 }
 
-int batch_step(cpsd_gpu_batch *b)
+int batch_step(cpsd_gpu_batch *b, bool first)
 {
     const int par = b->cells[0]->cur;
-    if (!b->gexec[par]) {
+    cudaGraphExec_t &ge = b->gexec[first][par];
+    if (!ge) {
         cudaGraph_t g = nullptr;
         std::vector<long long> before;
         for (auto *c : b->cells) before.push_back(c->nlaunch);
@@ -1574,7 +1618,9 @@ int batch_step(cpsd_gpu_batch *b)
         for (size_t i = 0; i < b->cells.size() && e == cudaSuccess && rc == CPSD_OK; ++i) {
             cpsd_gpu_ctx *c = b->cells[i];
             e = cudaStreamWaitEvent(c->st, b->ev[0], 0);
+            c->with_sf = first;
             if (e == cudaSuccess) rc = one_step(c);
+            c->with_sf = true;
             c->cur = par;  // capture launched nothing: undo the buffer flip
             if (e == cudaSuccess) e = cudaEventRecord(b->ev[1 + i], c->st);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(b->st, b->ev[1 + i], 0);
@@ -1585,18 +1631,18 @@ int batch_step(cpsd_gpu_batch *b)
             captured += b->cells[i]->nlaunch - before[i];
             b->cells[i]->nlaunch = before[i];
         }
-        b->graph_launches = (int)captured;
+        b->graph_launches[first] = (int)captured;
         if (rc || e != cudaSuccess || e2 != cudaSuccess) {
             if (g) cudaGraphDestroy(g);
             (void)cudaGetLastError();
             return rc ? rc : CPSD_ERR_CUDA;
         }
-        e = cudaGraphInstantiate(&b->gexec[par], g, 0);
+        e = cudaGraphInstantiate(&ge, g, 0);
         cudaGraphDestroy(g);
         CK(e);
     }
-    CK(cudaGraphLaunch(b->gexec[par], b->st));
-    b->nlaunch += b->graph_launches;
+    CK(cudaGraphLaunch(ge, b->st));
+    b->nlaunch += b->graph_launches[first];
     for (auto *c : b->cells) c->cur ^= 1;
     return CPSD_OK;
 }
@@ -2133,7 +2179,7 @@ int cpsd_gpu_batch_run(cpsd_gpu_batch *b, int inner, double *E, double *deltae, 
         CK(cudaMemcpyAsync(c->Edev, E + 10 * i, sizeof(double), cudaMemcpyHostToDevice, b->st));
     }
     for (int it = 0; it < inner; ++it) {
-        int rc = batch_step(b);
+        int rc = batch_step(b, it == 0);
         if (rc) return rc;
     }
     // energies per cell on its own stream after the batch's steps
@@ -2247,8 +2293,12 @@ int cpsd_gpu_create(const cpsd_gpu_params *p, const int *masker1, cpsd_gpu_ctx *
     c->ldc = h.npw_pad;
     CK(cudaSetDevice(p->device));
     c->sms = device_sms();
-    CK(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking));
-    CK(cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking));
+    // the side stream's blocks (projector products) take the SM slots that the
+    // density -> potential -> V psi chain leaves
+    int lowest = 0, highest = 0;
+    CK(cudaDeviceGetStreamPriorityRange(&lowest, &highest));
+    CK(cudaStreamCreateWithPriority(&c->st, cudaStreamNonBlocking, highest));
+    CK(cudaStreamCreateWithPriority(&c->st2, cudaStreamNonBlocking, lowest));
     CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&c->ev_sf, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&c->ev_side, cudaEventDisableTiming));
