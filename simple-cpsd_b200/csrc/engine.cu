@@ -213,6 +213,7 @@ struct FftOps {
     virtual void fwd_z_store(const Geom &g, const void *Tb, cx<double> *out, long ldo, double scale,
                              int nb, cudaStream_t s) = 0;
     virtual void fwd_z_sd(const Geom &g, const void *Tb, const ZEpilogue &e, int nb, cudaStream_t s) = 0;
+    virtual void z_potential(const Geom &g, void *Tb, const ZPotArgs &a, cudaStream_t s) = 0;
     virtual void plane(int mode, const Geom &g, void *Tb, const PlaneArgs &a, int nchunks, cudaStream_t s) = 0;
     virtual int plane_ctas_per_sm(int mode) const = 0;  // resident CTAs of a plane pass
     virtual int plane_ctas_per_plane(int mode) const = 0;  // CTAs sharing one z plane (row split)
@@ -365,6 +366,7 @@ struct FftOpsT final : FftOps {
         int dev = 0, optin = 0;
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+        static_assert(zpot_smem_bytes<T, NF>() <= 48 << 10, "no opt-in shared memory");
         CK(cudaFuncSetAttribute(inv_z_kernel<T, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem));
         CK(cudaFuncSetAttribute(fwd_z_kernel<T, NF, ZEPI_STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem));
         CK(cudaFuncSetAttribute(fwd_z_kernel<T, NF, ZEPI_SD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem));
@@ -450,6 +452,12 @@ struct FftOpsT final : FftOps {
         constexpr int CPB = kThreads / Line<NF>::P;
         dim3 grid((unsigned)cdiv(g.ncol, CPB), (unsigned)nb);
         fwd_z_kernel<T, NF, ZEPI_SD><<<grid, kThreads, zsmem, s>>>(g, (const cx<T> *)Tb, e, tw);
+    }
+    void z_potential(const Geom &g, void *Tb, const ZPotArgs &a, cudaStream_t s) override
+    {
+        constexpr int CPB = kZPotThreads / Line<NF>::P;
+        z_potential_kernel<T, NF><<<(unsigned)cdiv(g.ncol, CPB), kZPotThreads, zpot_smem_bytes<T, NF>(), s>>>(
+            g, (cx<T> *)Tb, a, tw);
     }
     void plane(int mode, const Geom &g, void *Tb, const PlaneArgs &a, int nchunks, cudaStream_t s) override
     {
@@ -654,7 +662,7 @@ struct cpsd_gpu_ctx {
     double *r1 = nullptr, *r2 = nullptr, *fion = nullptr;
     void *Tb = nullptr, *Taux = nullptr;
     double *rho_part = nullptr, *dn = nullptr, *xcp = nullptr, *xce = nullptr, *rfwd = nullptr, *Vr = nullptr;
-    cx<double> *dng = nullptr, *vall = nullptr, *sfac = nullptr, *Vg = nullptr, *proj = nullptr;
+    cx<double> *dng = nullptr, *vall = nullptr, *sfac = nullptr, *proj = nullptr;
     cx<double> *ex1 = nullptr, *ex2 = nullptr, *ex3 = nullptr;
     double *beta = nullptr, *coefT = nullptr, *Mov = nullptr, *gws = nullptr, *lag = nullptr;
     double *lmd = nullptr, *hml = nullptr, *Edev = nullptr, *red = nullptr;
@@ -1164,19 +1172,17 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
             c->nlaunch += 1;
             mark(c, 3);
         }
-        // rho(G), cpsd.c:198-205
+        // the density's forward plane pass, cpsd.c:198-205
         PlaneArgs pf{};
         pf.rin = c->rfwd;
         c->fft->plane(PM_FWDREAL, c->g, c->Taux, pf, 1, s); c->nlaunch += 1;
-        c->fft->fwd_z_store(c->g, c->Taux, c->dng, c->ldc, 1.0, 1, s); c->nlaunch += 1;
         mark(c, 4);
         if (fork && with_sf)
             CK(cudaStreamWaitEvent(s, c->ev_sf, 0));
         else if (!fork)
             issue_sf(c, side);
-        // V(G), cpsd.c:373-379
-        vg_kernel<<<(unsigned)cdiv(c->npw, 128), 128, 0, s>>>(c->npw, c->vall, c->dng, c->vc, c->scal2, c->Vg);
-        c->nlaunch += 1;
+        // rho(G) on the sphere and V(G), back to the potential's columns (cpsd.c:205, 373-379)
+        c->fft->z_potential(c->g, c->Taux, ZPotArgs{c->vall, c->vc, c->scal2, c->dng}, s); c->nlaunch += 1;
         if (c->move && c->nion > 0) {  // local, k-space and real-space Ewald forces
             ForceArgs fa{};
             fa.npw = c->npw;
@@ -1208,7 +1214,6 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
         }
         mark(c, 5);
         // V_loc + V_H to real space, plus xc per spin (cpsd.c:380-388)
-        c->fft->inv_z(c->g, c->Vg, c->ldc, c->Taux, 1, s); c->nlaunch += 1;
         PlaneArgs pv{};
         pv.rout = c->Vr;
         pv.xadd = c->xcp;
@@ -2409,7 +2414,6 @@ int cpsd_gpu_create(const cpsd_gpu_params *p, const int *masker1, cpsd_gpu_ctx *
     CK(ar.alloc(&c->dng, P));
     CK(ar.alloc(&c->vall, P));
     CK(ar.alloc(&c->sfac, P));
-    CK(ar.alloc(&c->Vg, P));
     CK(ar.alloc(&c->ex1, (size_t)std::max(nion, 1) * c->nh));
     CK(ar.alloc(&c->ex2, (size_t)std::max(nion, 1) * c->n));
     CK(ar.alloc(&c->ex3, (size_t)std::max(nion, 1) * c->n));

@@ -257,6 +257,122 @@ fwd_z_kernel(Geom g, const cx<T> *__restrict__ Tb, ZEpilogue e, Twiddles<T> tw)
     }
 }
 
+// ------------------------------------------------------------ z_potential
+// The density's columns (after the plane pass) -> rho(G), V(G) = vall / omega +
+// rho(G) vc (ccpsdv3/cpsd.c:205, 373-379) -> the potential's columns, all of one
+// column at a time, so the forward and inverse kz lines and the product in
+// between are one launch (three before).  One field has few columns (181 at
+// 64^3, 697 at 128^3): CTAs of 64 threads spread them over the SMs; bound by
+// latency.  Against the three launches the chain rho(r) -> V(r) is 5.7 us
+// shorter at 64^3 (26.7 -> 21 us) and 6.5 us at 128^3.
+constexpr int kZPotThreads = 64;
+
+template <typename T, int NF>
+constexpr int zpot_tile_elems()  // the column tile, the exchange buffers or the rows
+{
+    constexpr int CPB = kZPotThreads / Line<NF>::P;
+    constexpr int TILE = (CPB * (NF + 1) > NF * (CPB + 1)) ? CPB * (NF + 1) : NF * (CPB + 1);
+    constexpr int XB = CPB * group_stride<T, NF>();
+    return TILE > XB ? TILE : XB;
+}
+template <typename T, int NF>
+constexpr size_t zpot_smem_bytes()
+{
+    constexpr int CPB = kZPotThreads / Line<NF>::P;
+    return sizeof(cx<T>) * ((size_t)zpot_tile_elems<T, NF>() + CPB * (NF + 1) + 2 * NF);
+}
+
+struct ZPotArgs {
+    const cx<double> *vall;
+    const double *vc;
+    double scal2;
+    cx<double> *dng;  // out: rho(G) on the sphere
+};
+
+template <typename T, int NF>
+__global__ void __launch_bounds__(kZPotThreads) z_potential_kernel(Geom g, cx<T> *__restrict__ Tb, ZPotArgs a,
+                                                                   Twiddles<T> tw)
+{
+    using L = Line<NF>;
+    constexpr int P = L::P, Q = L::Q, U = L::U, CPB = kZPotThreads / P;
+    constexpr int RS = NF + 1, CS = CPB + 1;
+    constexpr int XS = group_stride<T, NF>();
+    extern __shared__ unsigned char smem_raw[];
+    cx<T> *tile = reinterpret_cast<cx<T> *>(smem_raw);
+    cx<T> *vrow = tile + zpot_tile_elems<T, NF>();  // V(G) of the columns, zero off the sphere
+    cx<T> *twf = vrow + CPB * RS, *twi = twf + NF;
+    const int c0 = blockIdx.x * CPB;
+    const int grp = threadIdx.x / P, t = threadIdx.x % P;
+    const int c = c0 + grp;
+    for (int i = threadIdx.x; i < NF; i += kZPotThreads) {
+        twf[i] = tw.n_fwd[i];
+        twi[i] = tw.n_inv[i];
+    }
+    for (int i = threadIdx.x; i < CPB * RS; i += kZPotThreads) vrow[i] = cx<T>{0, 0};
+    for (int idx = threadIdx.x; idx < NF * CPB; idx += kZPotThreads) {
+        const int z = idx / CPB, cl = idx % CPB;
+        if (c0 + cl < g.ncol)
+            cp_async_cx(tile + z * CS + cl, Tb + (long)z * g.ncol + c0 + cl);
+        else
+            tile[z * CS + cl] = cx<T>{0, 0};
+    }
+    cp_async_commit_all();
+    cp_async_wait_all();
+    __syncthreads();
+    cx<T> v[Q];
+#pragma unroll
+    for (int m = 0; m < Q; ++m) v[m] = tile[L::in_index(t, m) * CS + grp];
+    __syncthreads();  // every column read: the exchange buffers overwrite the tile
+    line_fft<NF, -1, T>(v, t, tile + grp * XS, twf);
+    __syncthreads();
+    cx<T> *row = tile + grp * RS;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int s = 0; s < P; ++s) row[L::out_index(t, u, s)] = v[u * P + s];
+    __syncwarp();
+    if (c < g.ncol) {
+        const int pe = g.col_ptr[c + 1];
+        for (int p0 = g.col_ptr[c] + t; p0 < pe; p0 += 4 * P) {
+            int kk[4];
+            cx<double> va[4];
+            double k[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int p = p0 + u * P;
+                kk[u] = -1;
+                if (p < pe) {
+                    kk[u] = g.pt_k[p];
+                    va[u] = a.vall[p];
+                    k[u] = a.vc[p];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (kk[u] < 0) continue;
+                const cx<T> F = row[kk[u]];
+                const cx<double> d{(double)F.x, (double)F.y};
+                a.dng[p0 + u * P] = d;
+                vrow[grp * RS + kk[u]] = cx<T>{(T)(va[u].x * a.scal2 + d.x * k[u]), (T)(va[u].y * a.scal2 + d.y * k[u])};
+            }
+        }
+    }
+    __syncthreads();  // every row read: the exchange buffers overwrite them
+#pragma unroll
+    for (int m = 0; m < Q; ++m) v[m] = vrow[grp * RS + L::in_index(t, m)];
+    line_fft<NF, +1, T>(v, t, tile + grp * XS, twi);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int s = 0; s < P; ++s) tile[L::out_index(t, u, s) * CS + grp] = v[u * P + s];
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < NF * CPB; idx += kZPotThreads) {
+        const int z = idx / CPB, cl = idx % CPB;
+        if (c0 + cl < g.ncol) Tb[(long)z * g.ncol + c0 + cl] = tile[z * CS + cl];
+    }
+}
+
 // ------------------------------------------------------------------ plane
 enum { PM_DENSITY = 0, PM_APPLYV = 1, PM_INVREAL = 2, PM_FWDREAL = 3 };
 

@@ -64,7 +64,7 @@ CPSD_D cx<double> strfac_point(cx<double> e1, cx<double> e2, cx<double> e3)
 }
 
 // ------------------------------------------------------------ local psp, projectors
-// ccpsdv3/cpsd.c:224-245 (s, vall), :260-286 (projectors), :373-379 (V(G))
+// ccpsdv3/cpsd.c:224-245 (s, vall), :260-286 (projectors)
 struct VlocArgs {
     int npw, npw_pad, n, nh, nion;
     const int *pt_i, *pt_j, *pt_k;
@@ -112,17 +112,6 @@ __global__ void vloc_proj_kernel(VlocArgs a)
     }
     a.s[p] = s;
     a.vall[p] = vall;
-}
-
-// V(G) = vall / omega + dng vc (cpsd.c:373-379), once the density is known
-__global__ void vg_kernel(int npw, const cx<double> *__restrict__ vall, const cx<double> *__restrict__ dng,
-                          const double *__restrict__ vc, double scal2, cx<double> *__restrict__ Vg)
-{
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= npw) return;
-    const cx<double> v = vall[p], d = dng[p];
-    const double k = vc[p];
-    Vg[p] = cx<double>{v.x * scal2 + d.x * k, v.y * scal2 + d.y * k};
 }
 
 // ------------------------------------------------------------ ion forces
