@@ -311,6 +311,16 @@ constexpr int group_stride()
 }
 
 // ---------------------------------------------------------------------------
+// Programmatic dependent launch: a kernel of the step's main chain may be
+// scheduled while its predecessor still runs; it stages its constant tables
+// (twiddles) and waits here for the predecessor's results.  Every thread of
+// every such kernel waits before it touches anything a kernel wrote, so a
+// finished predecessor implies finished predecessors of its own.  Both are
+// no-ops in a launch without the attribute.
+CPSD_D void chain_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+CPSD_D void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------
 // error flags written by kernels (host reads them after a step)
 enum : int {
     CPSD_DEVFLAG_BAD_INDEX = 1,

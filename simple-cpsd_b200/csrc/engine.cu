@@ -203,18 +203,37 @@ cudaError_t upload(DevArena &ar, X **d, const std::vector<X> &h)
     return cudaMemcpy(*d, h.data(), h.size() * sizeof(X), cudaMemcpyHostToDevice);
 }
 
+// Launch; chain: as a programmatic dependent of the stream's last kernel (see
+// chain_wait), for kernels that call chain_wait.
+template <typename K, typename... A>
+void launch(K *kernel, dim3 grid, int threads, size_t smem, cudaStream_t s, bool chain, const A &...args)
+{
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = chain ? 1 : 0;
+    (void)cudaLaunchKernelEx(&cfg, kernel, args...);  // errors: cudaGetLastError of the phase
+}
+
 // ------------------------------------------------------------ transform engines
 struct FftOps {
     virtual ~FftOps() = default;
     virtual size_t elem() const = 0;
     // span: see HostGeom::span
     virtual int init(DevArena &ar, int KX, int ncol, int span) = 0;
-    virtual void inv_z(const Geom &g, const cx<double> *psi, long ldp, void *Tb, int nb, cudaStream_t s) = 0;
+    // chain: see launch()
+    virtual void inv_z(const Geom &g, const cx<double> *psi, long ldp, void *Tb, int nb, cudaStream_t s, bool chain) = 0;
     virtual void fwd_z_store(const Geom &g, const void *Tb, cx<double> *out, long ldo, double scale,
                              int nb, cudaStream_t s) = 0;
     virtual void fwd_z_sd(const Geom &g, const void *Tb, const ZEpilogue &e, int nb, cudaStream_t s) = 0;
-    virtual void z_potential(const Geom &g, void *Tb, const ZPotArgs &a, cudaStream_t s) = 0;
-    virtual void plane(int mode, const Geom &g, void *Tb, const PlaneArgs &a, int nchunks, cudaStream_t s) = 0;
+    virtual void z_potential(const Geom &g, void *Tb, const ZPotArgs &a, cudaStream_t s, bool chain) = 0;
+    virtual void plane(int mode, const Geom &g, void *Tb, const PlaneArgs &a, int nchunks, cudaStream_t s, bool chain) = 0;
     virtual int plane_ctas_per_sm(int mode) const = 0;  // resident CTAs of a plane pass
     virtual int plane_ctas_per_plane(int mode) const = 0;  // CTAs sharing one z plane (row split)
     virtual int plane_bands(int mode) const = 0;           // bands a band pass transforms together
@@ -323,7 +342,7 @@ struct FftOpsT final : FftOps {
     }
 
     template <int MODE>
-    void bands(const Geom &g, void *Tb, const PlaneArgs &a, int nchunks, cudaStream_t s)
+    void bands(const Geom &g, void *Tb, const PlaneArgs &a, int nchunks, cudaStream_t s, bool chain)
     {
         PairArgs pa{};
         pa.chunk_b0 = a.chunk_b0;
@@ -334,7 +353,7 @@ struct FftOpsT final : FftOps {
         pa.stage = a.chunk_bands > 2 && pair[MODE].sm_stage != 0;
         const size_t sm = pa.stage ? pair[MODE].sm_stage : pair[MODE].sm;
         with_pair<MODE>([&](auto *k) {
-            k<<<dim3(NF, (unsigned)nchunks), PairCfg<T, NF, MODE>::NT, sm, s>>>(g, (cx<T> *)Tb, pa, ptw);
+            launch(k, dim3(NF, (unsigned)nchunks), PairCfg<T, NF, MODE>::NT, sm, s, chain, g, (cx<T> *)Tb, pa, ptw);
         });
     }
 
@@ -417,24 +436,24 @@ struct FftOpsT final : FftOps {
 
     // occ 1: the two-CTA build (128 registers a thread), occ 0: one CTA per SM
     template <int MODE>
-    void launch_plane(dim3 grid, int nt, const Geom &g, void *Tb, const PlaneArgs &a, cudaStream_t s)
+    void launch_plane(dim3 grid, int nt, const Geom &g, void *Tb, const PlaneArgs &a, cudaStream_t s, bool chain)
     {
         if constexpr (plane_has_two_cta_build<NF, MODE>())
             if (occ[MODE]) {
                 dim3 g2 = grid;
                 g2.z = plane_row_split<NF, MODE, 2>();  // the density pass's row halves
                 const size_t sm = (g2.z > 1) ? psmem_split : psmem[MODE];
-                plane_kernel<T, NF, MODE, 2><<<g2, nt, sm, s>>>(g, (cx<T> *)Tb, a, tw);
+                launch(plane_kernel<T, NF, MODE, 2>, g2, nt, sm, s, chain, g, (cx<T> *)Tb, a, tw);
                 return;
             }
-        plane_kernel<T, NF, MODE, 1><<<grid, nt, psmem[MODE], s>>>(g, (cx<T> *)Tb, a, tw);
+        launch(plane_kernel<T, NF, MODE, 1>, grid, nt, psmem[MODE], s, chain, g, (cx<T> *)Tb, a, tw);
     }
 
-    void inv_z(const Geom &g, const cx<double> *psi, long ldp, void *Tb, int nb, cudaStream_t s) override
+    void inv_z(const Geom &g, const cx<double> *psi, long ldp, void *Tb, int nb, cudaStream_t s, bool chain) override
     {
         constexpr int CPB = kThreads / Line<NF>::P;
         dim3 grid((unsigned)cdiv(g.ncol, CPB), (unsigned)nb);
-        inv_z_kernel<T, NF><<<grid, kThreads, zsmem, s>>>(g, psi, ldp, (cx<T> *)Tb, tw);
+        launch(inv_z_kernel<T, NF>, grid, kThreads, zsmem, s, chain, g, psi, ldp, (cx<T> *)Tb, tw);
     }
     void fwd_z_store(const Geom &g, const void *Tb, cx<double> *out, long ldo, double scale, int nb,
                      cudaStream_t s) override
@@ -453,27 +472,27 @@ struct FftOpsT final : FftOps {
         dim3 grid((unsigned)cdiv(g.ncol, CPB), (unsigned)nb);
         fwd_z_kernel<T, NF, ZEPI_SD><<<grid, kThreads, zsmem, s>>>(g, (const cx<T> *)Tb, e, tw);
     }
-    void z_potential(const Geom &g, void *Tb, const ZPotArgs &a, cudaStream_t s) override
+    void z_potential(const Geom &g, void *Tb, const ZPotArgs &a, cudaStream_t s, bool chain) override
     {
         constexpr int CPB = kZPotThreads / Line<NF>::P;
-        z_potential_kernel<T, NF><<<(unsigned)cdiv(g.ncol, CPB), kZPotThreads, zpot_smem_bytes<T, NF>(), s>>>(
-            g, (cx<T> *)Tb, a, tw);
+        launch(z_potential_kernel<T, NF>, dim3((unsigned)cdiv(g.ncol, CPB)), kZPotThreads, zpot_smem_bytes<T, NF>(), s,
+               chain, g, (cx<T> *)Tb, a, tw);
     }
-    void plane(int mode, const Geom &g, void *Tb, const PlaneArgs &a, int nchunks, cudaStream_t s) override
+    void plane(int mode, const Geom &g, void *Tb, const PlaneArgs &a, int nchunks, cudaStream_t s, bool chain) override
     {
         const dim3 grid(NF, (unsigned)nchunks);
         const int nt = plane_threads<T, NF>(mode);
         switch (mode) {
         case PM_DENSITY:
-            if (pair[PM_DENSITY].ok) return bands<PM_DENSITY>(g, Tb, a, nchunks, s);
-            if constexpr (kOneBand) launch_plane<PM_DENSITY>(grid, nt, g, Tb, a, s);
+            if (pair[PM_DENSITY].ok) return bands<PM_DENSITY>(g, Tb, a, nchunks, s, chain);
+            if constexpr (kOneBand) launch_plane<PM_DENSITY>(grid, nt, g, Tb, a, s, chain);
             break;
         case PM_APPLYV:
-            if (pair[PM_APPLYV].ok) return bands<PM_APPLYV>(g, Tb, a, nchunks, s);
-            if constexpr (kOneBand) launch_plane<PM_APPLYV>(grid, nt, g, Tb, a, s);
+            if (pair[PM_APPLYV].ok) return bands<PM_APPLYV>(g, Tb, a, nchunks, s, chain);
+            if constexpr (kOneBand) launch_plane<PM_APPLYV>(grid, nt, g, Tb, a, s, chain);
             break;
-        case PM_INVREAL: launch_plane<PM_INVREAL>(grid, nt, g, Tb, a, s); break;
-        default: launch_plane<PM_FWDREAL>(grid, nt, g, Tb, a, s); break;
+        case PM_INVREAL: launch_plane<PM_INVREAL>(grid, nt, g, Tb, a, s, chain); break;
+        default: launch_plane<PM_FWDREAL>(grid, nt, g, Tb, a, s, chain); break;
         }
     }
     int plane_bands(int mode) const override { return mode < 2 && pair[mode].ok ? 2 : 1; }
@@ -603,6 +622,7 @@ struct cpsd_gpu_ctx {
     // so that its copy to the host can start during the rest of the step
     cudaEvent_t ev_dn = nullptr;
     bool rec_dn = false;
+    bool in_batch = false;  // the step is being captured as one of a batch's cells
     bool with_sf = true;  // the step forms the structure factors and projectors
     cudaStream_t cs = nullptr;  // the stream the GEMM helpers launch on
     unsigned *ticket = nullptr;  // CTAs of the running small_overlap_kernel that are done
@@ -894,20 +914,22 @@ const double *Mblk(cpsd_gpu_ctx *c, int ms, int which)
 bool small_cell(const cpsd_gpu_ctx *c) { return c->ne0 <= kLagSmallMax; }
 
 template <int MODE, int MT>
-int launch_small(cpsd_gpu_ctx *c, const SmallArgs &a)
+int launch_small(cpsd_gpu_ctx *c, const SmallArgs &a, bool chain)
 {
     cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = kSmCluster;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3((unsigned)a.splits, (unsigned)c->ispin);
     cfg.blockDim = dim3(kSmThreads);
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.dynamicSmemBytes = small_smem_bytes<MODE, MT>(c->ne0);
     cfg.stream = c->cs;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = chain ? 2 : 1;
     CK(cudaLaunchKernelEx(&cfg, small_overlap_kernel<MODE, MT>, a));
     c->nlaunch += 1;
     return CPSD_OK;
@@ -915,7 +937,7 @@ int launch_small(cpsd_gpu_ctx *c, const SmallArgs &a)
 
 // A'WB of every spin's bands (small.cuh), MODE SM_LAGRANGE with a.lag set
 template <int MODE>
-int small_overlaps(cpsd_gpu_ctx *c, SmallArgs a, const double *A, const double *B)
+int small_overlaps(cpsd_gpu_ctx *c, SmallArgs a, const double *A, const double *B, bool chain = false)
 {
     a.K = 2 * c->npw_pad;
     a.ld = 2L * c->npw_pad;
@@ -930,10 +952,10 @@ int small_overlaps(cpsd_gpu_ctx *c, SmallArgs a, const double *A, const double *
     // at least four k-steps of 8 reals per warp, at most a CTA per SM
     a.splits = kSmCluster * (int)std::min<long>(kSmMaxClusters, std::max<long>(1, cdiv(a.K / 8, 4L * kSmWarps * kSmCluster)));
     switch (cdiv(c->ne0, 8)) {
-    case 1: return launch_small<MODE, 1>(c, a);
-    case 2: return launch_small<MODE, 2>(c, a);
-    case 3: return launch_small<MODE, 3>(c, a);
-    default: return launch_small<MODE, 4>(c, a);
+    case 1: return launch_small<MODE, 1>(c, a, chain);
+    case 2: return launch_small<MODE, 2>(c, a, chain);
+    case 3: return launch_small<MODE, 3>(c, a, chain);
+    default: return launch_small<MODE, 4>(c, a, chain);
     }
 }
 
@@ -957,7 +979,7 @@ int band_products(cpsd_gpu_ctx *c, const double *A, const double *B, double *con
 
 // Out_j = beta Out_j + alpha sum_l mat_ms[l + j m] In_l over the bands of each spin
 void band_rotation(cpsd_gpu_ctx *c, double alpha, const double *const *mat, const double *In, double beta, double *Out,
-                   int which = 0)
+                   int which = 0, bool chain = false)
 {
     const long ldr = 2L * c->npw_pad;
     if (small_cell(c)) {
@@ -976,10 +998,10 @@ void band_rotation(cpsd_gpu_ctx *c, double alpha, const double *const *mat, cons
         // a warp per 16 reals of the rows, up to two CTAs per SM
         const dim3 grid((unsigned)std::min<long>(2L * c->sms, cdiv(a.K / 16, kSmWarps)), (unsigned)c->ispin);
         switch (cdiv(c->ne0, 8)) {
-        case 1: small_nn_kernel<1><<<grid, kSmThreads, 0, c->cs>>>(a); break;
-        case 2: small_nn_kernel<2><<<grid, kSmThreads, 0, c->cs>>>(a); break;
-        case 3: small_nn_kernel<3><<<grid, kSmThreads, 0, c->cs>>>(a); break;
-        default: small_nn_kernel<4><<<grid, kSmThreads, 0, c->cs>>>(a); break;
+        case 1: launch(small_nn_kernel<1>, grid, kSmThreads, 0, c->cs, chain, a); break;
+        case 2: launch(small_nn_kernel<2>, grid, kSmThreads, 0, c->cs, chain, a); break;
+        case 3: launch(small_nn_kernel<3>, grid, kSmThreads, 0, c->cs, chain, a); break;
+        default: launch(small_nn_kernel<4>, grid, kSmThreads, 0, c->cs, chain, a); break;
         }
         c->nlaunch += 1;
         return;
@@ -1104,6 +1126,15 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
     // density pass instead (beside the small transforms; at the start they
     // would compete with it).  128^3 / 64 ions: 84 us a step of the side stream.
     const bool with_sf = c->with_sf || c->move || c->bp;
+    // The main chain's kernels are programmatic dependents of one another
+    // where the stream's last operation is such a kernel: not behind a copy,
+    // an event record (phase timing, rec_dn) or a join with the side stream.
+    // For one cell up to 64^3 (64^3, 16 bands, ten steps: 861 -> 806 us, FP32
+    // transforms 804 -> 743; 24 bands of a 32 bohr box 3.01 -> 2.86 ms): at
+    // 128^3 a waiting block of a band pass takes a whole SM from the side
+    // stream (32 bands 3.18 -> 3.33 ms, 128 bands 23.3 -> 23.6 ms), and a
+    // batch's other cells fill the gaps anyway (12 cells 8.51 -> 8.68 ms).
+    const bool chain = fork && !c->bp && c->n <= 64 && !c->in_batch;
     if (phase == 0) {
         if (with_sf) CK(copy_positions(c, s));
         auto side_work = [&]() -> int {
@@ -1126,7 +1157,7 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
         mark(c, 0);
         // psi(G) -> psi(r) and the density, cpsd.c:177-194
         if (nbl > 0) {
-            c->fft->inv_z(c->g, c1 + (long)lo * c->ldc, c->ldc, c->Tb, nbl, s);
+            c->fft->inv_z(c->g, c1 + (long)lo * c->ldc, c->ldc, c->Tb, nbl, s, chain && !with_sf);
             c->nlaunch += 1;
         }
         mark(c, 1);
@@ -1137,7 +1168,7 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
         pa.ne0 = (c->ispin == 2) ? std::max(0, c->ne0 - lo) : nbl;
         const int ch0 = c->bp ? c->nchunk_bp[0] : c->nchunk0, ch1 = c->bp ? c->nchunk_bp[1] : c->nchunk1;
         if (ch0 + ch1 > 0) {
-            c->fft->plane(PM_DENSITY, c->g, c->Tb, pa, ch0 + ch1, s);
+            c->fft->plane(PM_DENSITY, c->g, c->Tb, pa, ch0 + ch1, s, chain);
             c->nlaunch += 1;
         }
         if (fork && !with_sf) {
@@ -1152,7 +1183,7 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
             CK(cudaGetLastError());
             return CPSD_OK;
         }
-        density_xc_kernel<<<(unsigned)cdiv(c->n3, 256), 256, 0, s>>>(xa); c->nlaunch += 1;
+        launch(density_xc_kernel, dim3((unsigned)cdiv(c->n3, 256)), 256, 0, s, chain, xa); c->nlaunch += 1;
         if (c->rec_dn) {
             // while capturing, an external record: a plain one would only be a
             // dependency inside the graph, invisible to a wait outside it (the
@@ -1175,14 +1206,14 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
         // the density's forward plane pass, cpsd.c:198-205
         PlaneArgs pf{};
         pf.rin = c->rfwd;
-        c->fft->plane(PM_FWDREAL, c->g, c->Taux, pf, 1, s); c->nlaunch += 1;
+        c->fft->plane(PM_FWDREAL, c->g, c->Taux, pf, 1, s, chain && !c->rec_dn); c->nlaunch += 1;
         mark(c, 4);
         if (fork && with_sf)
             CK(cudaStreamWaitEvent(s, c->ev_sf, 0));
         else if (!fork)
             issue_sf(c, side);
         // rho(G) on the sphere and V(G), back to the potential's columns (cpsd.c:205, 373-379)
-        c->fft->z_potential(c->g, c->Taux, ZPotArgs{c->vall, c->vc, c->scal2, c->dng}, s); c->nlaunch += 1;
+        c->fft->z_potential(c->g, c->Taux, ZPotArgs{c->vall, c->vc, c->scal2, c->dng}, s, chain && !with_sf); c->nlaunch += 1;
         if (c->move && c->nion > 0) {  // local, k-space and real-space Ewald forces
             ForceArgs fa{};
             fa.npw = c->npw;
@@ -1218,7 +1249,7 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
         pv.rout = c->Vr;
         pv.xadd = c->xcp;
         pv.nout = c->ispin;
-        c->fft->plane(PM_INVREAL, c->g, c->Taux, pv, 1, s); c->nlaunch += 1;
+        c->fft->plane(PM_INVREAL, c->g, c->Taux, pv, 1, s, chain && !c->move); c->nlaunch += 1;
         mark(c, 6);
         if (!fork) {
             int rc = issue_knl(c, side, c1, c2, lo, nbl);
@@ -1232,7 +1263,7 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
             pp.chunk_bands = c->v_bands;
             pp.V = c->Vr;
             pp.ne0 = (c->ispin == 2) ? std::max(0, c->ne0 - lo) : nbl;
-            c->fft->plane(PM_APPLYV, c->g, c->Tb, pp, c->nchunk_v, s); c->nlaunch += 1;
+            c->fft->plane(PM_APPLYV, c->g, c->Tb, pp, c->nchunk_v, s, chain); c->nlaunch += 1;
         }
         mark(c, 8);
         if (fork) CK(cudaStreamWaitEvent(s, c->ev_side, 0));  // kinetic + nonlocal c2 is in place
@@ -1287,11 +1318,11 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
     if (small_cell(c)) {  // overlaps and solver in one launch
         SmallArgs a{};
         a.lag = la;
-        int rc = small_overlaps<SM_LAGRANGE>(c, a, (const double *)c2, (const double *)c1);
+        int rc = small_overlaps<SM_LAGRANGE>(c, a, (const double *)c2, (const double *)c1, chain && !c->mlp);
         if (rc) return rc;
         mark(c, 10);
         mark(c, 11);
-        band_rotation(c, c->dte, lmds, (const double *)c1, 1.0, (double *)c2);
+        band_rotation(c, c->dte, lmds, (const double *)c1, 1.0, (double *)c2, 0, chain);
         mark(c, 12);
         CK(cudaGetLastError());
         c->cur ^= 1;
@@ -1564,16 +1595,16 @@ int cpsd_fft_run_full(int n, int dir, const Geom &g, double *grid, cx<double> *p
     }
     if (dir > 0) {
         if (!e->inv_ok) return CPSD_ERR_GRID;
-        e->ops->inv_z(g, packed, g.npw, Taux, 1, st);
+        e->ops->inv_z(g, packed, g.npw, Taux, 1, st, false);
         PlaneArgs pv{};
         pv.rout = grid;
         pv.nout = 1;
-        e->ops->plane(PM_INVREAL, g, Taux, pv, 1, st);
+        e->ops->plane(PM_INVREAL, g, Taux, pv, 1, st, false);
     } else {
         if (!e->fwd_ok) return CPSD_ERR_GRID;
         PlaneArgs pf{};
         pf.rin = grid;
-        e->ops->plane(PM_FWDREAL, g, Taux, pf, 1, st);
+        e->ops->plane(PM_FWDREAL, g, Taux, pf, 1, st, false);
         e->ops->fwd_z_store(g, Taux, packed, g.npw, 1.0, 1, st);
     }
     CK(cudaGetLastError());
@@ -1624,7 +1655,9 @@ int batch_step(cpsd_gpu_batch *b, bool first)
             cpsd_gpu_ctx *c = b->cells[i];
             e = cudaStreamWaitEvent(c->st, b->ev[0], 0);
             c->with_sf = first;
+            c->in_batch = true;
             if (e == cudaSuccess) rc = one_step(c);
+            c->in_batch = false;
             c->with_sf = true;
             c->cur = par;  // capture launched nothing: undo the buffer flip
             if (e == cudaSuccess) e = cudaEventRecord(b->ev[1 + i], c->st);

@@ -117,6 +117,8 @@ inv_z_kernel(Geom g, const cx<double> *__restrict__ psi, long ldp, cx<T> *__rest
     cx<T> *row = tile + grp * RS;
     for (int k = t; k < NF; k += P) row[k] = cx<T>{0, 0};
     __syncwarp();
+    chain_wait();
+    chain_start();
     if (c < g.ncol) {
         // four points per lane in flight: their loads before their stores
         const cx<double> *src = psi + (long)b * ldp;
@@ -192,6 +194,8 @@ fwd_z_kernel(Geom g, const cx<T> *__restrict__ Tb, ZEpilogue e, Twiddles<T> tw)
     const int c = c0 + grp;
     cx<T> *twz = tile + z_tile_elems<T, NF>();  // W_NF^-m staged once per CTA
     for (int i = threadIdx.x; i < NF; i += kThreads) twz[i] = tw.n_fwd[i];
+    chain_wait();
+    chain_start();
     // the column tile by cp.async: every element of a thread in flight at once
     const cx<T> *src = Tb + (long)b * NF * g.ncol;
     for (int idx = threadIdx.x; idx < NF * CPB; idx += kThreads) {
@@ -309,6 +313,8 @@ __global__ void __launch_bounds__(kZPotThreads) z_potential_kernel(Geom g, cx<T>
         twi[i] = tw.n_inv[i];
     }
     for (int i = threadIdx.x; i < CPB * RS; i += kZPotThreads) vrow[i] = cx<T>{0, 0};
+    chain_wait();
+    chain_start();
     for (int idx = threadIdx.x; idx < NF * CPB; idx += kZPotThreads) {
         const int z = idx / CPB, cl = idx % CPB;
         if (c0 + cl < g.ncol)
@@ -487,6 +493,8 @@ plane_kernel(Geom g, cx<T> *__restrict__ Tb, PlaneArgs a, Twiddles<T> twg)
     cx<T> *Y = stage + stage_elems<T>(STAGE ? MODE : -1, g.ncol);  // [KX][YS]
     cx<T> *xball = Y + KX * YS;                                     // group exchange buffers
     for (int i = threadIdx.x; i < TwLayout<NF>::total; i += NT) tws[i] = twg.n_inv[i];
+    chain_wait();
+    chain_start();
     const Twiddles<T> tw = Twiddles<T>::template at<NF>(tws);
     __syncthreads();
     // DENSITY: each lane owns the same (row, x) points for every band, so the

@@ -364,6 +364,8 @@ CPSD_D void dirac_vosko(int ispin, double nup_in, double ndn_in, double rho0, do
 
 __global__ void density_xc_kernel(XcArgs a)
 {
+    chain_wait();
+    chain_start();
     const long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= a.n3) return;
     double d[2] = {0.0, 0.0}, r0 = 0.0, r1 = 0.0;

@@ -297,6 +297,8 @@ pair_kernel(Geom g, cx<T> *__restrict__ Tb, PairArgs a, const cx<T> *__restrict_
     void *xb = C::SPLIT ? (void *)(reinterpret_cast<T *>(Y + 2 * KX * YS) + gr * C::GS)
                         : (void *)(Y + 2 * KX * YS + gr * C::GS);
     for (int i = threadIdx.x; i < PairTw<NF>::total; i += NT) tws[i] = twg[i];
+    chain_wait();
+    chain_start();
     const cx<T> *twi = tws + PairTw<NF>::inv, *twd = tws + PairTw<NF>::dif;
 
     const int z = blockIdx.x;

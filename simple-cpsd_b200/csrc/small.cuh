@@ -240,6 +240,8 @@ __global__ void __launch_bounds__(kSmThreads, 1) small_overlap_kernel(const __gr
     extern __shared__ __align__(16) double sm_raw[];
     __shared__ unsigned slot[kSmWarps][4];
     __shared__ int last;
+    chain_wait();
+    chain_start();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = lane >> 2, q = lane & 3;
     const int ms = blockIdx.y, m = a.m[ms];
     const double *__restrict__ A = a.A[ms], *__restrict__ B = a.B[ms];
@@ -408,6 +410,8 @@ struct SmallNNArgs {
 template <int MT>
 __global__ void __launch_bounds__(kSmThreads) small_nn_kernel(const __grid_constant__ SmallNNArgs a)
 {
+    chain_wait();
+    chain_start();
     const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
     const int ms = blockIdx.y, m = a.m[ms];
     const double *__restrict__ mat = a.mat[ms], *__restrict__ in = a.in[ms];
