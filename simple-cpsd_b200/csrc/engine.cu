@@ -630,7 +630,7 @@ struct cpsd_gpu_ctx {
     bool lag_tile_ok = false;  // the tiled solver can run on this device for these bands
     // tuning (cpsd_gpu_set_tuning / cpsd_gpu_autotune): split-K target of the
     // TN products, density chunk capacity and the model's chunk counts
-    int tn_ctas = 2;
+    int tn_ctas = 4;
     int dens_cap = 0;
     int dens_model[2] = {0, 0};
     // band-parallel SD (cpsd_gpu_set_band_range): this context transforms and
@@ -767,7 +767,21 @@ int plan_v_chunks(cpsd_gpu_ctx *c, int n0, int n1)
     return CPSD_OK;
 }
 
-// Split-K plan of a batch of weighted TN products: about two CTAs per SM
+// The shared memory of the FP64 product kernels (above the 48 KB default).
+cudaError_t allow_dm_smem()
+{
+    const void *tn[2] = {(const void *)gemm_tn_dmma_kernel<true>, (const void *)gemm_tn_dmma_kernel<false>};
+    const void *nn[2] = {(const void *)gemm_nn_dmma_kernel<true>, (const void *)gemm_nn_dmma_kernel<false>};
+    for (int q = 0; q < 2; ++q) {
+        cudaError_t e = cudaFuncSetAttribute(tn[q], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDmTnSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(nn[q], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDmNnSmem);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+// Split-K plan of a batch of weighted TN products: four CTAs per SM by default
+// (what is resident; 128 bands, three overlaps: two 188 us, four 136 us)
 // (sms: the device's SM count), each split at least 64 reals, partials
 // within ws_elems.
 struct TnPlan {
@@ -775,11 +789,16 @@ struct TnPlan {
     int kchunk;
 };
 
-TnPlan tn_plan(int M, int N, int K, int nprod, bool tc, size_t ws_elems, int sms, int ctas_per_sm = 2)
+TnPlan tn_plan(int M, int N, int K, int nprod, bool tc, size_t ws_elems, int sms, int ctas_per_sm = 4, unsigned sym = 0)
 {
     const int tm = tc ? kTcM : kDmT, tn = tc ? kTcN : kDmT, bk = tc ? kTcBK : kDmK;
-    const long tiles = cdiv(M, tm) * cdiv(N, tn) * nprod;
-    long splits = std::max<long>(1, cdiv((long)ctas_per_sm * sms, tiles));
+    if (tc) ctas_per_sm = std::min(ctas_per_sm, 2);  // one is resident
+    long tiles = cdiv(M, tm) * cdiv(N, tn) * nprod;
+    // tiles below the diagonal of a product read by its upper triangle are not formed
+    for (int q = 0; q < nprod && !tc; ++q)
+        if ((sym >> q) & 1) tiles -= cdiv(M, tm) * (cdiv(M, tm) - 1) / 2;
+    // at most ctas_per_sm on every SM: one CTA too many would make a second round
+    long splits = std::max<long>(1, (long)ctas_per_sm * sms / tiles);
     splits = std::min<long>(splits, std::max<long>(1, K / 64));
     while ((size_t)splits * M * N * nprod > ws_elems && splits > 1) --splits;
     const int kchunk = (int)(cdiv(cdiv(K, splits), bk) * bk);
@@ -791,9 +810,9 @@ TnPlan tn_plan(int M, int N, int K, int nprod, bool tc, size_t ws_elems, int sms
 // reduction.  Returns the number of launches.
 int launch_tn(int M, int N, int K, int nprod, const double *const *A, long lda, const double *const *B, long ldb,
               const double *w, double alpha, double beta, double *const *C, long ldc, bool tc, double *ws,
-              size_t ws_elems, int *err, cudaStream_t s, int ctas_per_sm = 2)
+              size_t ws_elems, int *err, cudaStream_t s, int ctas_per_sm = 4, unsigned sym = 0)
 {
-    const TnPlan pl = tn_plan(M, N, K, nprod, tc, ws_elems, device_sms(), ctas_per_sm);
+    const TnPlan pl = tn_plan(M, N, K, nprod, tc, ws_elems, device_sms(), ctas_per_sm, sym);
     TnBatch bt{};
     for (int q = 0; q < nprod; ++q) {
         bt.A[q] = A[q];
@@ -807,10 +826,16 @@ int launch_tn(int M, int N, int K, int nprod, const double *const *A, long lda, 
         tc_gemm_tn_kernel<<<grid, kTcThreads, kTcSmem, s>>>(M, N, K, lda, ldb, w, pl.kchunk, bt, ws, err);
     } else {
         dim3 grid((unsigned)cdiv(M, kDmT), (unsigned)cdiv(N, kDmT), (unsigned)(pl.splits * nprod));
-        gemm_tn_dmma_kernel<<<grid, kDmThreads, 0, s>>>(M, N, K, lda, ldb, w, pl.kchunk, bt, ws);
+        bt.sym = sym;
+        bool v2 = (lda % 2) == 0 && (ldb % 2) == 0;
+        for (int q = 0; q < nprod; ++q) v2 = v2 && ((uintptr_t)A[q] % 16) == 0 && ((uintptr_t)B[q] % 16) == 0;
+        if (v2)
+            gemm_tn_dmma_kernel<true><<<grid, kDmThreads, kDmTnSmem, s>>>(M, N, K, lda, ldb, w, pl.kchunk, bt, ws);
+        else
+            gemm_tn_dmma_kernel<false><<<grid, kDmThreads, kDmTnSmem, s>>>(M, N, K, lda, ldb, w, pl.kchunk, bt, ws);
     }
-    splitk_reduce_kernel<<<(unsigned)cdiv((long)M * N * nprod * 32, 256), 256, 0, s>>>(M, N, ldc, ws, alpha, beta,
-                                                                                       bt);
+    splitk_reduce_kernel<<<(unsigned)(cdiv((long)M * N, kRedOut) * nprod), kRedOut * kRedGroups, 0, s>>>(
+        M, N, ldc, ws, alpha, beta, bt);
     return 2;
 }
 
@@ -836,13 +861,13 @@ bool tc_product(const cpsd_gpu_ctx *c, int which, int M, int N)
 // and its GEMM mode includes that product.
 int gemm_tn_batch(cpsd_gpu_ctx *c, int M, int N, int K, int nprod, const double *const *A, long lda,
                   const double *const *B, long ldb, const double *w, double alpha, double beta,
-                  double *const *C, long ldc, int which = 0)
+                  double *const *C, long ldc, int which = 0, unsigned sym = 0)
 {
     if (M <= 0 || N <= 0 || nprod <= 0) return CPSD_OK;
     if (nprod > kTnMaxProd) return CPSD_ERR_ARG;
     const bool tc = tc_product(c, which, M, N);
     c->nlaunch += launch_tn(M, N, K, nprod, A, lda, B, ldb, w, alpha, beta, C, ldc, tc, c->gws, c->gemm_ws_elems,
-                            c->flags + 2, c->cs, c->tn_ctas);
+                            c->flags + 2, c->cs, c->tn_ctas, sym);
     return CPSD_OK;
 }
 
@@ -862,7 +887,7 @@ int overlaps3(cpsd_gpu_ctx *c, int m, int K, long ld, const double *C2, const do
     const bool tc = (c->gemm_mode & TN_OVERLAPS) != 0 && c->precision == CPSD_PREC_MIXED;
     const bool fits = m > 0 && m <= kTcM && (ld % 2) == 0 && K % 2 == 0 && ((uintptr_t)C1 % 16) == 0 &&
                       ((uintptr_t)C2 % 16) == 0;
-    if (!tc || !fits) return gemm_tn_batch(c, m, m, K, 3, As, ld, Bs, ld, c->w, 1.0, 0.0, Cs, m, TN_OVERLAPS);
+    if (!tc || !fits) return gemm_tn_batch(c, m, m, K, 3, As, ld, Bs, ld, c->w, 1.0, 0.0, Cs, m, TN_OVERLAPS, 0b101u);  // C2'WC2 and C1'WC1: one triangle is read (cpsd.c:426-436)
     const long mm = (long)m * m;
     long splits = std::min<long>(c->sms, std::max<long>(1, K / 64));
     while ((size_t)splits * 3 * mm > c->gemm_ws_elems && splits > 1) --splits;
@@ -878,7 +903,8 @@ int overlaps3(cpsd_gpu_ctx *c, int m, int K, long ld, const double *C2, const do
     }
     bt.nprod = 3;
     bt.splits = (int)splits;
-    splitk_reduce_kernel<<<(unsigned)cdiv(mm * 3 * 32, 256), 256, 0, c->cs>>>(m, m, m, c->gws, 1.0, 0.0, bt);
+    splitk_reduce_kernel<<<(unsigned)(cdiv(mm, kRedOut) * 3), kRedOut * kRedGroups, 0, c->cs>>>(m, m, m, c->gws, 1.0,
+                                                                                              0.0, bt);
     c->nlaunch += 2;
     return CPSD_OK;
 }
@@ -896,7 +922,13 @@ void gemm_nn(cpsd_gpu_ctx *c, int NJ, int K, int L, double alpha, const double *
                                                                 c->flags + 2);
     } else {
         dim3 grid((unsigned)cdiv(K, kDmT), (unsigned)cdiv(NJ, kDmT));
-        gemm_nn_dmma_kernel<<<grid, kDmThreads, 0, c->cs>>>(NJ, K, L, alpha, Mat, ldm, B, ldb, beta, Out, ldo);
+        const bool v2 = (ldm % 2) == 0 && (ldb % 2) == 0 && ((uintptr_t)Mat % 16) == 0 && ((uintptr_t)B % 16) == 0;
+        if (v2)
+            gemm_nn_dmma_kernel<true><<<grid, kDmThreads, kDmNnSmem, c->cs>>>(NJ, K, L, alpha, Mat, ldm, B, ldb, beta,
+                                                                             Out, ldo);
+        else
+            gemm_nn_dmma_kernel<false><<<grid, kDmThreads, kDmNnSmem, c->cs>>>(NJ, K, L, alpha, Mat, ldm, B, ldb, beta,
+                                                                              Out, ldo);
     }
     c->nlaunch += 1;
 }
@@ -959,8 +991,9 @@ int small_overlaps(cpsd_gpu_ctx *c, SmallArgs a, const double *A, const double *
     }
 }
 
-// C_ms[i][j] = <A_i|B_j> over the bands of each spin (Gamma-point weights)
-int band_products(cpsd_gpu_ctx *c, const double *A, const double *B, double *const *C, int which = 0)
+// C_ms[i][j] = <A_i|B_j> over the bands of each spin (Gamma-point weights);
+// upper: the caller reads i <= j only
+int band_products(cpsd_gpu_ctx *c, const double *A, const double *B, double *const *C, int which = 0, bool upper = false)
 {
     if (small_cell(c)) {
         SmallArgs a{};
@@ -971,7 +1004,9 @@ int band_products(cpsd_gpu_ctx *c, const double *A, const double *B, double *con
     for (int ms = 0; ms < c->ispin; ++ms) {
         const int m = ms ? c->ne1 : c->ne0;
         const long off = (long)(ms ? c->ne0 : 0) * ldr;
-        const int rc = gemm_tn(c, m, m, 2 * c->npw_pad, A + off, ldr, B + off, ldr, c->w, 1.0, 0.0, C[ms], m, which);
+        const double *Ao = A + off, *Bo = B + off;
+        const int rc = gemm_tn_batch(c, m, m, 2 * c->npw_pad, 1, &Ao, ldr, &Bo, ldr, c->w, 1.0, 0.0, &C[ms], m, which,
+                                     upper ? 1u : 0u);
         if (rc) return rc;
     }
     return CPSD_OK;
@@ -1513,7 +1548,7 @@ int energies(cpsd_gpu_ctx *c, int inner)
     const cx<double> *c2 = c->cbuf[c->cur], *c1 = c->cbuf[c->cur ^ 1];
     FinalArgs fa{};
     double *Mh[2] = {(double *)Mblk(c, 0, 3), (double *)Mblk(c, 1, 3)};
-    int rc = band_products(c, (const double *)c1, (const double *)c->cpsi, Mh);
+    int rc = band_products(c, (const double *)c1, (const double *)c->cpsi, Mh, 0, true);
     if (rc) return rc;
     fa.Mh[0] = Mh[0];
     fa.Mh[1] = Mh[1];
@@ -2492,6 +2527,7 @@ int cpsd_gpu_create(const cpsd_gpu_params *p, const int *masker1, cpsd_gpu_ctx *
     CK(ar.alloc(&c->pM, (size_t)c->ispin * c->ne0 * c->ne0));
     CK(ar.alloc(&c->pstats, (size_t)3 * nb));
     CK(ar.alloc(&c->py, (size_t)nb * kShells));
+    CK(allow_dm_smem());
     if (small_cell(c.get())) {
         auto allow = [&](auto one, auto lag, size_t so, size_t sl) {
             cudaError_t e = cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)so);
@@ -3582,6 +3618,7 @@ int noalloc_scratch(double **out)
         double *p = nullptr;
         CK(cudaGetSymbolAddress((void **)&p, g_overlap_scratch));
         CK(cudaFuncSetAttribute(tc_gemm_tn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
+        CK(allow_dm_smem());
         g_noalloc_base[dev] = p;
     }
     *out = g_noalloc_base[dev];
@@ -3603,6 +3640,8 @@ int cpsd_overlap_tn(int method, int M, int N, int K, const double *A, long lda, 
     const bool tc = method != CPSD_GEMM_FP64;
     if (tc)
         CK(cudaFuncSetAttribute(tc_gemm_tn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
+    else
+        CK(allow_dm_smem());
     const size_t cap = std::max<size_t>((size_t)M * N, (size_t)4 << 20);
     const TnPlan pl = tn_plan(M, N, K, 1, tc, cap, device_sms());
     struct Scratch {

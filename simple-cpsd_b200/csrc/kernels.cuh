@@ -452,26 +452,37 @@ struct TnBatch {
     const double *B[kTnMaxProd];
     double *C[kTnMaxProd];
     int nprod, splits;
+    unsigned sym;  // products read by their upper triangle only (bit per product)
 };
 
-// C_prod[i*ldc+j] = alpha * sum_s part[prod][s][i][j] (+ beta C): one warp
-// per output, lanes stride over the splits, then a fixed xor butterfly, so
-// the order of the additions (and the bits of the result) never changes.
-__global__ void splitk_reduce_kernel(int M, int N, long ldc, const double *__restrict__ part, double alpha,
-                                     double beta, const __grid_constant__ TnBatch bt)
+// C_prod[i*ldc+j] = alpha * sum_s part[prod][s][i][j] (+ beta C): a block takes
+// 32 neighbouring outputs (256-byte reads of every split's partials) and eight
+// interleaved groups of splits, then adds the groups in order: the order of
+// the additions (and the bits of the result) never changes.  128 bands, three
+// products of 59 splits: 24 us as a warp per output with lanes over the splits
+// (an 8-byte read per 32-byte sector), 9 us here.
+constexpr int kRedOut = 32, kRedGroups = 8;
+__global__ void __launch_bounds__(kRedOut * kRedGroups)
+splitk_reduce_kernel(int M, int N, long ldc, const double *__restrict__ part, double alpha,
+                     double beta, const __grid_constant__ TnBatch bt)
 {
-    const long wid = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    const long MN = (long)M * N;
-    if (wid >= MN * bt.nprod) return;  // whole warps leave together
-    const int prod = (int)(wid / MN);
-    const long e = wid % MN;
-    const double *p = part + (long)prod * bt.splits * MN + e;
+    __shared__ double sh[kRedGroups][kRedOut];
+    const long MN = (long)M * N, nblk = (MN + kRedOut - 1) / kRedOut;
+    const int x = threadIdx.x % kRedOut, y = threadIdx.x / kRedOut;
+    const int prod = (int)(blockIdx.x / nblk);
+    const long e = (blockIdx.x % nblk) * kRedOut + x;
+    const bool ok = e < MN && !(((bt.sym >> prod) & 1) && e / N > e % N);  // below the diagonal: not formed
     double s = 0.0;
-    for (int q = lane; q < bt.splits; q += 32) s += p[(long)q * MN];
+    if (ok) {
+        const double *p = part + (long)prod * bt.splits * MN + e;
+#pragma unroll 4
+        for (int q = y; q < bt.splits; q += kRedGroups) s += p[(long)q * MN];
+    }
+    sh[y][x] = s;
+    __syncthreads();
+    if (y == 0 && ok) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) {
+        for (int k = 1; k < kRedGroups; ++k) s += sh[k][x];
         const int i = (int)(e / N), j = (int)(e % N);
         double *c = bt.C[prod] + (long)i * ldc + j;
         *c = alpha * s + (beta == 0.0 ? 0.0 : beta * *c);
@@ -483,15 +494,25 @@ __global__ void splitk_reduce_kernel(int M, int N, long ldc, const double *__res
 // products, FP64 sums): the split-K weighted TN partials above and the
 // back-projection NN product (the reference's dgemm('N','N') on
 // column-major psi blocks, cpsd.c:483-488).  A CTA of four warps owns a 64x64 output
-// tile, each warp a 32x32 quadrant of 4x4 fragments of 8x8.  A shared tile
-// holds 16 values of the contraction index per row; MMA step s (0..3) feeds
-// fragment k-slot q with tile column 4q+s, so one lane's four values for a
-// tile are a contiguous 32-byte run (two 16-byte loads).  The next tile is
-// fetched into registers while the current one is multiplied: two shared
-// buffers, one barrier per tile.  Row strides keep every shared access free
-// of bank conflicts: kDmS = 18 puts consecutive rows 9 16-byte units apart,
-// kDmSB = 65 (NN B tile, [l][k]) staggers the four k-slots by one bank.
-constexpr int kDmT = 64, kDmK = 16, kDmThreads = 128, kDmS = 18, kDmSB = 65;
+// tile, each warp a 32x32 quadrant of 4x4 fragments of 8x8, and walks the
+// contraction in slabs of 16 that arrive by cp.async, kDmStages - 1 slabs
+// ahead, with one barrier per slab.
+//
+// Bound: the FP64 pipe (an m8n8k4 occupies its quarter of the SM for 16 cycles,
+// the rate of 8 DFMAs; 27 cycles latency).  The former kernels fetched the next
+// slab through registers and multiplied the weights into it as it arrived, so
+// every slab waited for its loads (42-49 % of the pipe); here the weights
+// multiply the fragments.
+constexpr int kDmT = 64, kDmK = 16, kDmThreads = 128, kDmStages = 3;
+// TN: rows of 16 reals, 18 apart: consecutive rows sit 9 16-byte units apart, a
+// lane's pair of k-slots (tile columns 4q + 2h, +1) is one 16-byte load, free
+// of bank conflicts.
+constexpr int kDmS = 18;
+// NN: matrix rows 24 apart with k-slot q = tile columns 2q, 2q + 1 of each half,
+// operand rows of 64 columns 66 apart: both free of conflicts
+constexpr int kDmSA = 24, kDmSB = 66;
+constexpr size_t kDmTnSmem = sizeof(double) * kDmStages * (2 * kDmT * kDmS + kDmK / 2);
+constexpr size_t kDmNnSmem = sizeof(double) * kDmStages * (kDmT * kDmSA + kDmK * kDmSB);
 
 CPSD_D void dmma(double &d0, double &d1, double a, double b)
 {
@@ -500,62 +521,88 @@ CPSD_D void dmma(double &d0, double &d1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
+// n (0, 1 or 2) doubles to a pair in shared memory, the rest zero.  V2: the
+// source is 16-byte aligned (one 16-byte copy), else two 8-byte copies.
+template <bool V2>
+CPSD_D void cp_async_pair(double *dst, const double *src, int n)
+{
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if constexpr (V2) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(8 * n) : "memory");
+    } else {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n > 0 ? 8 : 0) : "memory");
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d + 8), "l"(n > 1 ? src + 1 : src),
+                     "r"(n > 1 ? 8 : 0) : "memory");
+    }
+}
+CPSD_D void dm_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+CPSD_D void dm_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 // part[prod][split][i][j] as above; grid (M tiles, N tiles, nprod * splits).
+// Products whose bit in bt.sym is set are read by their upper triangle only
+// (i <= j): their tiles below the diagonal are not formed.
+template <bool V2>
 __global__ void __launch_bounds__(kDmThreads, 4)
 gemm_tn_dmma_kernel(int M, int N, int K, long lda, long ldb, const double *__restrict__ w, int kchunk,
                     const __grid_constant__ TnBatch bt, double *__restrict__ part)
 {
-    __shared__ __align__(16) double As[2][kDmT * kDmS], Bs[2][kDmT * kDmS];
+    extern __shared__ __align__(16) double dm_sm[];
     const int prod = blockIdx.z / bt.splits, split = blockIdx.z % bt.splits;
+    if (((bt.sym >> prod) & 1) && blockIdx.x > blockIdx.y) return;
+    double *As = dm_sm, *Bs = As + kDmStages * kDmT * kDmS, *Ws = Bs + kDmStages * kDmT * kDmS;
     const double *__restrict__ A = bt.A[prod];
     const double *__restrict__ B = bt.B[prod];
     const int i0 = blockIdx.x * kDmT, j0 = blockIdx.y * kDmT;
     const int k0 = split * kchunk, k1 = min(K, k0 + kchunk);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wr = (warp >> 1) * 32, wc = (warp & 1) * 32, fr = lane >> 2, fq = lane & 3;
-    double ra[4][2], rb[4][2];
-    // loader: pass q moves reals (2p, 2p+1) of tile row e>>3, e = tid + 128q, p = e&7
-    auto fetch = [&](int kk) {
+    const int ns = k1 > k0 ? (k1 - k0 + kDmK - 1) / kDmK : 0;
+    // slab it: thread -> reals (2p, 2p+1) of rows row, row + 16, .. (p = tid & 7, row = tid >> 3)
+    auto issue = [&](int it) {
+        const int st = it % kDmStages, k = k0 + it * kDmK + 2 * (tid & 7);
+        const int n = min(2, max(0, k1 - k));
+        double *a = As + st * kDmT * kDmS + 2 * (tid & 7), *b = Bs + st * kDmT * kDmS + 2 * (tid & 7);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const int e = tid + kDmThreads * q, row = e >> 3, k = kk + 2 * (e & 7);
-            const int i = i0 + row, j = j0 + row;
-            const double wk = (w != nullptr && k < k1) ? w[k >> 1] : 1.0;  // k even: one weight per pair
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const bool ok = k + h < k1;
-                ra[q][h] = (ok && i < M) ? A[(long)i * lda + k + h] * wk : 0.0;
-                rb[q][h] = (ok && j < N) ? B[(long)j * ldb + k + h] : 0.0;
-            }
+            const int row = (tid >> 3) + 16 * q, i = i0 + row, j = j0 + row;
+            cp_async_pair<V2>(a + row * kDmS, n > 0 && i < M ? A + (long)i * lda + k : A, i < M ? n : 0);
+            cp_async_pair<V2>(b + row * kDmS, n > 0 && j < N ? B + (long)j * ldb + k : B, j < N ? n : 0);
+        }
+        if (w != nullptr && tid < kDmK / 2) {  // one weight per pair (k0 is even)
+            const int kw = k0 + it * kDmK + 2 * tid;
+            const uint32_t d = (uint32_t)__cvta_generic_to_shared(Ws + st * (kDmK / 2) + tid);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(w + (kw < k1 ? kw >> 1 : 0)),
+                         "r"(kw < k1 ? 8 : 0) : "memory");
         }
     };
-    auto stash = [&](int buf) {
+    if (w == nullptr && tid < kDmStages * kDmK / 2) Ws[tid] = 1.0;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int e = tid + kDmThreads * q, off = (e >> 3) * kDmS + 2 * (e & 7);
-            *reinterpret_cast<double2 *>(&As[buf][off]) = make_double2(ra[q][0], ra[q][1]);
-            *reinterpret_cast<double2 *>(&Bs[buf][off]) = make_double2(rb[q][0], rb[q][1]);
-        }
-    };
-    double acc[4][4][2] = {};
-    int buf = 0;
-    if (k0 < k1) {
-        fetch(k0);
-        stash(0);
+    for (int it = 0; it < kDmStages - 1; ++it) {
+        if (it < ns) issue(it);
+        dm_commit();
     }
-    __syncthreads();
-    for (int kk = k0; kk < k1; kk += kDmK) {
-        const bool more = kk + kDmK < k1;
-        if (more) fetch(kk + kDmK);
+    double acc[4][4][2] = {};
+    for (int it = 0; it < ns; ++it) {
+        dm_wait<kDmStages - 2>();
+        __syncthreads();  // slab it has landed for every thread; the slot of slab it - 1 is free
+        if (it + kDmStages - 1 < ns) issue(it + kDmStages - 1);
+        dm_commit();
+        const int st = it % kDmStages;
+        const double *as = As + st * kDmT * kDmS, *bs = Bs + st * kDmT * kDmS;
+        const double2 ww = *reinterpret_cast<const double2 *>(Ws + st * (kDmK / 2) + 2 * fq);
         // two halves of two k-steps each: one 16-byte fragment load per
         // operand row per half keeps the fragments in 32 registers
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
             double2 a[4], b[4];
+            const double wk = hh ? ww.y : ww.x;
 #pragma unroll
             for (int f = 0; f < 4; ++f) {
-                a[f] = *reinterpret_cast<const double2 *>(As[buf] + (wr + 8 * f + fr) * kDmS + 4 * fq + 2 * hh);
-                b[f] = *reinterpret_cast<const double2 *>(Bs[buf] + (wc + 8 * f + fr) * kDmS + 4 * fq + 2 * hh);
+                a[f] = *reinterpret_cast<const double2 *>(as + (wr + 8 * f + fr) * kDmS + 4 * fq + 2 * hh);
+                b[f] = *reinterpret_cast<const double2 *>(bs + (wc + 8 * f + fr) * kDmS + 4 * fq + 2 * hh);
+                a[f].x *= wk;
+                a[f].y *= wk;
             }
 #pragma unroll
             for (int fi = 0; fi < 4; ++fi)
@@ -566,10 +613,8 @@ gemm_tn_dmma_kernel(int M, int N, int K, long lda, long ldb, const double *__res
 #pragma unroll
                 for (int fj = 0; fj < 4; ++fj) dmma(acc[fi][fj][0], acc[fi][fj][1], a[fi].y, b[fj].y);
         }
-        if (more) stash(buf ^ 1);
-        __syncthreads();
-        buf ^= 1;
     }
+    dm_wait<0>();
     double *out = part + ((long)prod * bt.splits + split) * M * N;
 #pragma unroll
     for (int fi = 0; fi < 4; ++fi) {
@@ -587,59 +632,56 @@ gemm_tn_dmma_kernel(int M, int N, int K, long lda, long ldb, const double *__res
 
 // Out[j*ldo+k] = beta*Out + alpha * sum_l
 // Mat[l + j*ldm] * B[l*ldb + k]; grid x over 64-wide k tiles, y over j tiles.
-__global__ void __launch_bounds__(kDmThreads, 4)
+// V2: Mat, B and their strides are 16-byte aligned.
+template <bool V2>
+__global__ void __launch_bounds__(kDmThreads, 3)
 gemm_nn_dmma_kernel(int NJ, int K, int L, double alpha, const double *__restrict__ Mat, long ldm,
-                    const double *__restrict__ B, long ldb, double beta, double *__restrict__ Out, long ldo)
+                    const double *__restrict__ B, long ldb, double beta, double *Out, long ldo)
 {
-    __shared__ __align__(16) double Ms[2][kDmT * kDmS], Bs[2][kDmK * kDmSB];
+    extern __shared__ __align__(16) double dm_sm[];
+    double *Ms = dm_sm, *Bs = Ms + kDmStages * kDmT * kDmSA;
     const int k0 = blockIdx.x * kDmT, j0 = blockIdx.y * kDmT;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wr = (warp >> 1) * 32, wc = (warp & 1) * 32, fr = lane >> 2, fq = lane & 3;
-    double rm[4][2], rb[8];
-    auto fetch = [&](int l0) {
+    const int ns = (L + kDmK - 1) / kDmK;
+    auto issue = [&](int it) {
+        const int st = it % kDmStages, l0 = it * kDmK;
+        double *m = Ms + st * kDmT * kDmSA + 2 * (tid & 7), *b = Bs + st * kDmK * kDmSB + 2 * (tid & 31);
+        const int l = l0 + 2 * (tid & 7), n = min(2, max(0, L - l));
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {  // Mat: tile row j = e>>3, l pair (2p, 2p+1)
-            const int e = tid + kDmThreads * q, j = j0 + (e >> 3), l = l0 + 2 * (e & 7);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) rm[q][h] = (j < NJ && l + h < L) ? Mat[(long)j * ldm + l + h] : 0.0;
+        for (int q = 0; q < 4; ++q) {  // Mat: row j, reals l, l + 1
+            const int row = (tid >> 3) + 16 * q, j = j0 + row;
+            cp_async_pair<V2>(m + row * kDmSA, n > 0 && j < NJ ? Mat + (long)j * ldm + l : Mat, j < NJ ? n : 0);
         }
+        const int k = k0 + 2 * (tid & 31), nk = min(2, max(0, K - k));
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {  // B: tile row l = e>>6, column k = e&63
-            const int e = tid + kDmThreads * q, l = l0 + (e >> 6), k = k0 + (e & 63);
-            rb[q] = (l < L && k < K) ? B[(long)l * ldb + k] : 0.0;
-        }
-    };
-    auto stash = [&](int buf) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int e = tid + kDmThreads * q;
-            *reinterpret_cast<double2 *>(&Ms[buf][(e >> 3) * kDmS + 2 * (e & 7)]) = make_double2(rm[q][0], rm[q][1]);
-        }
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int e = tid + kDmThreads * q;
-            Bs[buf][(e >> 6) * kDmSB + (e & 63)] = rb[q];
+        for (int q = 0; q < 4; ++q) {  // B: row l, reals k, k + 1
+            const int row = (tid >> 5) + 4 * q, lb = l0 + row;
+            cp_async_pair<V2>(b + row * kDmSB, nk > 0 && lb < L ? B + (long)lb * ldb + k : B, lb < L ? nk : 0);
         }
     };
-    double acc[4][4][2] = {};
-    int buf = 0;
-    if (L > 0) {
-        fetch(0);
-        stash(0);
+#pragma unroll
+    for (int it = 0; it < kDmStages - 1; ++it) {
+        if (it < ns) issue(it);
+        dm_commit();
     }
-    __syncthreads();
-    for (int l0 = 0; l0 < L; l0 += kDmK) {
-        const bool more = l0 + kDmK < L;
-        if (more) fetch(l0 + kDmK);
+    double acc[4][4][2] = {};
+    for (int it = 0; it < ns; ++it) {
+        dm_wait<kDmStages - 2>();
+        __syncthreads();
+        if (it + kDmStages - 1 < ns) issue(it + kDmStages - 1);
+        dm_commit();
+        const int st = it % kDmStages;
+        const double *ms = Ms + st * kDmT * kDmSA, *bt = Bs + st * kDmK * kDmSB;
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {  // two k-steps per half, as in the TN kernel
+        for (int hh = 0; hh < 2; ++hh) {  // two k-steps per half: tile columns 8 hh + 2q, + 1
             double2 a[4];
 #pragma unroll
             for (int f = 0; f < 4; ++f)
-                a[f] = *reinterpret_cast<const double2 *>(Ms[buf] + (wr + 8 * f + fr) * kDmS + 4 * fq + 2 * hh);
+                a[f] = *reinterpret_cast<const double2 *>(ms + (wr + 8 * f + fr) * kDmSA + 8 * hh + 2 * fq);
 #pragma unroll
             for (int s2 = 0; s2 < 2; ++s2) {
-                const double *bs = Bs[buf] + (4 * fq + 2 * hh + s2) * kDmSB + wc + fr;
+                const double *bs = bt + (8 * hh + 2 * fq + s2) * kDmSB + wc + fr;
                 double b[4];
 #pragma unroll
                 for (int fj = 0; fj < 4; ++fj) b[fj] = bs[8 * fj];
@@ -650,25 +692,44 @@ gemm_nn_dmma_kernel(int NJ, int K, int L, double alpha, const double *__restrict
                         dmma(acc[fi][fj][0], acc[fi][fj][1], s2 ? a[fi].y : a[fi].x, b[fj]);
             }
         }
-        if (more) stash(buf ^ 1);
-        __syncthreads();
-        buf ^= 1;
     }
+    dm_wait<0>();
+    // every old value is read before any new one is stored (a row's stores
+    // would keep the next row's loads back)
+    const bool pairs = V2 && (ldo % 2) == 0 && ((uintptr_t)Out % 16) == 0;
+    double2 old[4][4];
 #pragma unroll
-    for (int fi = 0; fi < 4; ++fi) {
-        const int j = j0 + wr + 8 * fi + fr;
-        if (j >= NJ) continue;
+    for (int fi = 0; fi < 4; ++fi)
 #pragma unroll
-        for (int fj = 0; fj < 4; ++fj)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int k = k0 + wc + 8 * fj + 2 * fq + h;
-                if (k < K) {
-                    double *o = Out + (long)j * ldo + k;
-                    *o = alpha * acc[fi][fj][h] + (beta == 0.0 ? 0.0 : beta * *o);
+        for (int fj = 0; fj < 4; ++fj) {
+            const int j = j0 + wr + 8 * fi + fr, k = k0 + wc + 8 * fj + 2 * fq;
+            old[fi][fj] = make_double2(0.0, 0.0);
+            if (beta != 0.0 && j < NJ) {
+                const double *o = Out + (long)j * ldo + k;
+                if (pairs && k + 1 < K) {
+                    old[fi][fj] = *reinterpret_cast<const double2 *>(o);
+                } else {
+                    if (k < K) old[fi][fj].x = o[0];
+                    if (k + 1 < K) old[fi][fj].y = o[1];
                 }
             }
-    }
+        }
+#pragma unroll
+    for (int fi = 0; fi < 4; ++fi)
+#pragma unroll
+        for (int fj = 0; fj < 4; ++fj) {
+            const int j = j0 + wr + 8 * fi + fr, k = k0 + wc + 8 * fj + 2 * fq;
+            if (j >= NJ) continue;
+            double *o = Out + (long)j * ldo + k;
+            const double2 v = make_double2(alpha * acc[fi][fj][0] + (beta == 0.0 ? 0.0 : beta * old[fi][fj].x),
+                                           alpha * acc[fi][fj][1] + (beta == 0.0 ? 0.0 : beta * old[fi][fj].y));
+            if (pairs && k + 1 < K) {
+                *reinterpret_cast<double2 *>(o) = v;
+            } else {
+                if (k < K) o[0] = v.x;
+                if (k + 1 < K) o[1] = v.y;
+            }
+        }
 }
 
 // ------------------------------------------------------------ Lagrange multipliers
