@@ -385,7 +385,9 @@ enum { PM_DENSITY = 0, PM_APPLYV = 1, PM_INVREAL = 2, PM_FWDREAL = 3 };
 struct PlaneArgs {
     const int *chunk_b0;  // band range of blockIdx.y: [chunk_b0[y], chunk_b0[y+1])
     double *rho_part;     // DENSITY: [chunk][z][y][x] sums of psi^2
-    const double *V;      // APPLYV: [ispin][z][y][x] total local potential
+    // APPLYV: [ispin][z][y][x] total local potential; the FP32 transforms keep
+    // each value as a float pair, high and low part, in its 8 bytes
+    const double *V;
     int ne0;              // bands b >= ne0 use V of spin 1
     double *rout;         // INVREAL: rout[ms] = psi + xadd[ms], ms < nout
     const double *xadd;
@@ -619,13 +621,19 @@ plane_kernel(Geom g, cx<T> *__restrict__ Tb, PlaneArgs a, Twiddles<T> twg)
                                 const long o = (long)z * plane + (long)j * NF + 2 * m;
                                 for (int ms = 0; ms < a.nout; ++ms) {
                                     double *ro = a.rout + ms * NF * plane;
+                                    double2 r = make_double2((double)w.x, (double)w.y);
                                     if (a.xadd) {
-                                        const double *xa = a.xadd + ms * NF * plane;
-                                        ro[o] = (double)w.x + xa[o];
-                                        ro[o + 1] = (double)w.y + xa[o + 1];
+                                        const double2 xa =
+                                            *reinterpret_cast<const double2 *>(a.xadd + ms * NF * plane + o);
+                                        r.x += xa.x;
+                                        r.y += xa.y;
+                                    }
+                                    if constexpr (sizeof(T) == 4) {  // high and low parts (PlaneArgs::V)
+                                        const float hx = (float)r.x, hy = (float)r.y;
+                                        *reinterpret_cast<float4 *>(ro + o) =
+                                            make_float4(hx, (float)(r.x - (double)hx), hy, (float)(r.y - (double)hy));
                                     } else {
-                                        ro[o] = (double)w.x;
-                                        ro[o + 1] = (double)w.y;
+                                        *reinterpret_cast<double2 *>(ro + o) = r;
                                     }
                                 }
                             }

@@ -270,7 +270,7 @@ CPSD_D void pair_forward(cx<T> *v, int t, void *xb, const cx<T> *__restrict__ tw
 struct PairArgs {
     const int *chunk_b0;  // bands of blockIdx.y: [chunk_b0[y], chunk_b0[y+1])
     double *rho_part;     // DENSITY: [chunk][z][y][x] sums of psi^2
-    const double *V;      // APPLYV: [ispin][z][y][x] total local potential
+    const double *V;      // APPLYV: see PlaneArgs::V
     int ne0;              // bands b >= ne0 are spin 1's (V of spin 1; never paired with spin 0's)
     int stage;            // the next pair's columns are copied ahead into shared memory
 };
@@ -408,7 +408,19 @@ pair_kernel(Geom g, cx<T> *__restrict__ Tb, PairArgs a, const cx<T> *__restrict_
                     rho[it][q] += (double)v[q].y * (double)v[q].y;
                 }
             } else {
+                // FP32: psi V = psi V_hi + psi V_lo in FP32 (one rounding of the
+                // sum; V_hi + V_lo holds 48 bits of V): the products in FP64 took
+                // two conversions and a multiplication of the FP64 pipe each
+                // (128 bands at 128^3: 0.516 ms, 0.479 this way).
                 const double *V = a.V + ((b >= a.ne0) ? NF * plane : 0) + (long)z * plane + (long)(act ? j : 0) * NF;
+                auto times = [](cx<T> w, double v) {
+                    if constexpr (sizeof(T) == 4) {
+                        const float hi = __int_as_float(__double2loint(v)), lo = __int_as_float(__double2hiint(v));
+                        return cx<T>{fmaf(w.x, hi, w.x * lo), fmaf(w.y, hi, w.y * lo)};
+                    } else {
+                        return cx<T>{w.x * v, w.y * v};
+                    }
+                };
 #pragma unroll
                 for (int s = 0; s < P; ++s) {
                     if constexpr (U % 2 == 0) {
@@ -416,15 +428,13 @@ pair_kernel(Geom g, cx<T> *__restrict__ Tb, PairArgs a, const cx<T> *__restrict_
                         for (int u = 0; u < U; u += 2) {
                             const double2 vv = *reinterpret_cast<const double2 *>(V + L::out_index(t, u, s));
                             cx<T> &w0 = v[u * P + s], &w1 = v[(u + 1) * P + s];
-                            w0 = cx<T>{(T)((double)w0.x * vv.x), (T)((double)w0.y * vv.x)};
-                            w1 = cx<T>{(T)((double)w1.x * vv.y), (T)((double)w1.y * vv.y)};
+                            w0 = times(w0, vv.x);
+                            w1 = times(w1, vv.y);
                         }
                     } else {
 #pragma unroll
                         for (int u = 0; u < U; ++u) {
-                            const double vv = V[L::out_index(t, u, s)];
-                            cx<T> &w0 = v[u * P + s];
-                            w0 = cx<T>{(T)((double)w0.x * vv), (T)((double)w0.y * vv)};
+                            v[u * P + s] = times(v[u * P + s], V[L::out_index(t, u, s)]);
                         }
                     }
                 }
