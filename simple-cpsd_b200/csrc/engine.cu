@@ -249,7 +249,8 @@ struct FftOpsT final : FftOps {
     Twiddles<T> tw{};
     int KX = 0;
     size_t zsmem = 0;
-    size_t psmem[4] = {0, 0, 0, 0};
+    size_t psmem[4] = {0, 0, 0, 0};   // of the two-CTA build
+    size_t psmem1[4] = {0, 0, 0, 0};  // of the one-CTA build (0: does not fit, the other one runs)
     size_t psmem_split = 0;  // the row-split density build (no staged columns)
     bool hi_fits[4] = {false, false, false, false};  // the high-occupancy build's CTAs fit an SM
     int occ[4] = {0, 0, 0, 0};                       // plane build that runs, per mode
@@ -389,10 +390,13 @@ struct FftOpsT final : FftOps {
         CK(cudaFuncSetAttribute(inv_z_kernel<T, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem));
         CK(cudaFuncSetAttribute(fwd_z_kernel<T, NF, ZEPI_STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem));
         CK(cudaFuncSetAttribute(fwd_z_kernel<T, NF, ZEPI_SD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem));
-        for (int m = 0; m < 4; ++m) psmem[m] = plane_smem_bytes<T, NF>(m, KX, ncol);
-        psmem_split = plane_smem_bytes<T, NF>(PM_DENSITY, KX, 0);
-        for (int m = 0; m < 4; ++m)
+        for (int m = 0; m < 4; ++m) {
+            psmem[m] = plane_smem_bytes<T, NF>(m, KX, ncol, 2);
+            psmem1[m] = plane_smem_bytes<T, NF>(m, KX, ncol, 1);
             if ((int)psmem[m] > optin) psmem[m] = 0;  // mode unavailable for this sphere
+            if ((int)psmem1[m] > optin) psmem1[m] = 0;
+        }
+        psmem_split = plane_smem_bytes<T, NF>(PM_DENSITY, KX, 0, 2);
         // The limit is a per-kernel (process-wide) attribute shared by every
         // context on the device: set it to the device maximum, launch with
         // what this sphere needs.
@@ -420,6 +424,9 @@ struct FftOpsT final : FftOps {
         // lines in two CTAs: measured slower than the whole-plane build, so
         // it is only a candidate of the tuner
         if (plane_row_split<NF, PM_DENSITY, 2>() > 1) occ[PM_DENSITY] = 0;
+        // the single-field passes' build with twice the threads, where it has them
+        for (int m : {PM_INVREAL, PM_FWDREAL})
+            if (plane_threads<NF>(m, 1) > kThreads && psmem1[m]) occ[m] = 0;
         int rc = init_pair<PM_DENSITY>(ncol, optin);
         if (!rc) rc = init_pair<PM_APPLYV>(ncol, optin);
         return rc;
@@ -435,18 +442,19 @@ struct FftOpsT final : FftOps {
     }
 
     // occ 1: the two-CTA build (128 registers a thread), occ 0: one CTA per SM
+    // (where it fits)
     template <int MODE>
-    void launch_plane(dim3 grid, int nt, const Geom &g, void *Tb, const PlaneArgs &a, cudaStream_t s, bool chain)
+    void launch_plane(dim3 grid, const Geom &g, void *Tb, const PlaneArgs &a, cudaStream_t s, bool chain)
     {
         if constexpr (plane_has_two_cta_build<NF, MODE>())
-            if (occ[MODE]) {
+            if (occ[MODE] || !psmem1[MODE]) {
                 dim3 g2 = grid;
                 g2.z = plane_row_split<NF, MODE, 2>();  // the density pass's row halves
                 const size_t sm = (g2.z > 1) ? psmem_split : psmem[MODE];
-                launch(plane_kernel<T, NF, MODE, 2>, g2, nt, sm, s, chain, g, (cx<T> *)Tb, a, tw);
+                launch(plane_kernel<T, NF, MODE, 2>, g2, plane_threads<NF>(MODE, 2), sm, s, chain, g, (cx<T> *)Tb, a, tw);
                 return;
             }
-        launch(plane_kernel<T, NF, MODE, 1>, grid, nt, psmem[MODE], s, chain, g, (cx<T> *)Tb, a, tw);
+        launch(plane_kernel<T, NF, MODE, 1>, grid, plane_threads<NF>(MODE, 1), psmem1[MODE], s, chain, g, (cx<T> *)Tb, a, tw);
     }
 
     void inv_z(const Geom &g, const cx<double> *psi, long ldp, void *Tb, int nb, cudaStream_t s, bool chain) override
@@ -481,18 +489,17 @@ struct FftOpsT final : FftOps {
     void plane(int mode, const Geom &g, void *Tb, const PlaneArgs &a, int nchunks, cudaStream_t s, bool chain) override
     {
         const dim3 grid(NF, (unsigned)nchunks);
-        const int nt = plane_threads<T, NF>(mode);
         switch (mode) {
         case PM_DENSITY:
             if (pair[PM_DENSITY].ok) return bands<PM_DENSITY>(g, Tb, a, nchunks, s, chain);
-            if constexpr (kOneBand) launch_plane<PM_DENSITY>(grid, nt, g, Tb, a, s, chain);
+            if constexpr (kOneBand) launch_plane<PM_DENSITY>(grid, g, Tb, a, s, chain);
             break;
         case PM_APPLYV:
             if (pair[PM_APPLYV].ok) return bands<PM_APPLYV>(g, Tb, a, nchunks, s, chain);
-            if constexpr (kOneBand) launch_plane<PM_APPLYV>(grid, nt, g, Tb, a, s, chain);
+            if constexpr (kOneBand) launch_plane<PM_APPLYV>(grid, g, Tb, a, s, chain);
             break;
-        case PM_INVREAL: launch_plane<PM_INVREAL>(grid, nt, g, Tb, a, s, chain); break;
-        default: launch_plane<PM_FWDREAL>(grid, nt, g, Tb, a, s, chain); break;
+        case PM_INVREAL: launch_plane<PM_INVREAL>(grid, g, Tb, a, s, chain); break;
+        default: launch_plane<PM_FWDREAL>(grid, g, Tb, a, s, chain); break;
         }
     }
     int plane_bands(int mode) const override { return mode < 2 && pair[mode].ok ? 2 : 1; }
@@ -545,12 +552,12 @@ template <typename T>
 size_t plane_need_t(int n, int mode, int KX, int ncol)
 {
     switch (n) {
-    case 16: return plane_smem_bytes<T, 16>(mode, KX, ncol);
-    case 24: return plane_smem_bytes<T, 24>(mode, KX, ncol);
-    case 32: return plane_smem_bytes<T, 32>(mode, KX, ncol);
-    case 48: return plane_smem_bytes<T, 48>(mode, KX, ncol);
-    case 64: return plane_smem_bytes<T, 64>(mode, KX, ncol);
-    default: return plane_smem_bytes<T, 128>(mode, KX, ncol);
+    case 16: return plane_smem_bytes<T, 16>(mode, KX, ncol, 2);
+    case 24: return plane_smem_bytes<T, 24>(mode, KX, ncol, 2);
+    case 32: return plane_smem_bytes<T, 32>(mode, KX, ncol, 2);
+    case 48: return plane_smem_bytes<T, 48>(mode, KX, ncol, 2);
+    case 64: return plane_smem_bytes<T, 64>(mode, KX, ncol, 2);
+    default: return plane_smem_bytes<T, 128>(mode, KX, ncol, 2);
     }
 }
 
