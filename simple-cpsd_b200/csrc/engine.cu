@@ -632,7 +632,7 @@ struct cpsd_gpu_ctx {
     bool in_batch = false;  // the step is being captured as one of a batch's cells
     bool with_sf = true;  // the step forms the structure factors and projectors
     cudaStream_t cs = nullptr;  // the stream the GEMM helpers launch on
-    unsigned *ticket = nullptr;  // CTAs of the running small_overlap_kernel that are done
+    unsigned *ticket = nullptr;  // CTAs of the running small_overlap_kernel that are done, per block
     bool lag_tile = false;  // 4 x 4 tiled solver (<= 128 bands, 16-CTA clusters schedulable)
     bool lag_tile_ok = false;  // the tiled solver can run on this device for these bands
     // tuning (cpsd_gpu_set_tuning / cpsd_gpu_autotune): split-K target of the
@@ -952,32 +952,56 @@ const double *Mblk(cpsd_gpu_ctx *c, int ms, int which)
 // (FP64, or 3xTF32 on 128 x 128 ones), a reduction and a solver launch.
 bool small_cell(const cpsd_gpu_ctx *c) { return c->ne0 <= kLagSmallMax; }
 
-template <int MODE, int MT>
-int launch_small(cpsd_gpu_ctx *c, const SmallArgs &a, bool chain)
+template <int MODE, int MT, int NB, int CL>
+int launch_small_cl(cpsd_gpu_ctx *c, const SmallArgs &a, int problems, int blocks, bool chain)
 {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kSmCluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)a.splits, (unsigned)c->ispin);
+    int n = 0;
+    if (CL > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = CL;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
+    if (chain) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    cfg.gridDim = dim3((unsigned)a.splits, (unsigned)problems, (unsigned)blocks);
     cfg.blockDim = dim3(kSmThreads);
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.dynamicSmemBytes = small_smem_bytes<MODE, MT>(c->ne0);
+    cfg.dynamicSmemBytes = small_smem_bytes<MODE, MT, NB>(c->ne0);
     cfg.stream = c->cs;
     cfg.attrs = attr;
-    cfg.numAttrs = chain ? 2 : 1;
-    CK(cudaLaunchKernelEx(&cfg, small_overlap_kernel<MODE, MT>, a));
+    cfg.numAttrs = n;
+    CK(cudaLaunchKernelEx(&cfg, small_overlap_kernel<MODE, MT, NB, CL>, a));
     c->nlaunch += 1;
     return CPSD_OK;
 }
 
-// A'WB of every spin's bands (small.cuh), MODE SM_LAGRANGE with a.lag set
-template <int MODE>
-int small_overlaps(cpsd_gpu_ctx *c, SmallArgs a, const double *A, const double *B, bool chain = false)
+bool small_clusters(int K) { return K / 8 > kSmNoClusterSteps; }
+
+template <int MODE, int MT, int NB>
+int launch_small(cpsd_gpu_ctx *c, const SmallArgs &a, int problems, int blocks, bool chain)
 {
+    return small_clusters(a.K) ? launch_small_cl<MODE, MT, NB, kSmCluster>(c, a, problems, blocks, chain)
+                               : launch_small_cl<MODE, MT, NB, 1>(c, a, problems, blocks, chain);
+}
+
+// CTAs along k of a small product: at least four k-steps of 8 reals per warp,
+// about a CTA per SM over all blocks
+int small_splits(int K, int blocks)
+{
+    if (!small_clusters(K)) return (int)std::max<long>(1, std::min<long>(kSmMaxClusters, cdiv(K / 8, 4L * kSmWarps)));
+    const long need = cdiv(K / 8, 4L * kSmWarps * kSmCluster);
+    return kSmCluster * (int)std::max<long>(1, std::min<long>(std::max(1, kSmMaxClusters / blocks), need));
+}
+
+// The three overlaps of every spin and the Lagrange solver (small.cuh)
+int small_overlaps(cpsd_gpu_ctx *c, const LagArgs &la, const double *C2, const double *C1, bool chain)
+{
+    SmallArgs a{};
+    a.lag = la;
     a.K = 2 * c->npw_pad;
     a.ld = 2L * c->npw_pad;
     a.w = c->w;
@@ -985,17 +1009,129 @@ int small_overlaps(cpsd_gpu_ctx *c, SmallArgs a, const double *A, const double *
     a.ticket = c->ticket;
     for (int ms = 0; ms < c->ispin; ++ms) {
         a.m[ms] = ms ? c->ne1 : c->ne0;
-        a.A[ms] = A + (ms ? c->ne0 : 0) * a.ld;
-        a.B[ms] = B + (ms ? c->ne0 : 0) * a.ld;
+        a.A[ms] = C2 + (ms ? c->ne0 : 0) * a.ld;
+        a.B[ms] = C1 + (ms ? c->ne0 : 0) * a.ld;
     }
-    // at least four k-steps of 8 reals per warp, at most a CTA per SM
-    a.splits = kSmCluster * (int)std::min<long>(kSmMaxClusters, std::max<long>(1, cdiv(a.K / 8, 4L * kSmWarps * kSmCluster)));
+    a.splits = small_splits(a.K, 1);
     switch (cdiv(c->ne0, 8)) {
-    case 1: return launch_small<MODE, 1>(c, a, chain);
-    case 2: return launch_small<MODE, 2>(c, a, chain);
-    case 3: return launch_small<MODE, 3>(c, a, chain);
-    default: return launch_small<MODE, 4>(c, a, chain);
+    case 1: return launch_small<SM_LAGRANGE, 1, 1>(c, a, c->ispin, 1, chain);
+    case 2: return launch_small<SM_LAGRANGE, 2, 2>(c, a, c->ispin, 1, chain);
+    case 3: return launch_small<SM_LAGRANGE, 3, 3>(c, a, c->ispin, 1, chain);
+    default: return launch_small<SM_LAGRANGE, 4, 4>(c, a, c->ispin, 1, chain);
     }
+}
+
+constexpr size_t kSmProjSmem = 160 << 10;
+
+// The small-cell kernels' shared memory; the attribute is the kernel's, shared
+// by every context of the device, so it is set to the most any needs.
+template <int MODE, int MT, int NB>
+cudaError_t allow_small()
+{
+    const int sm = (int)small_smem_bytes<MODE, MT, NB>(kLagSmallMax);
+    const cudaError_t e = cudaFuncSetAttribute(small_overlap_kernel<MODE, MT, NB, kSmCluster>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(small_overlap_kernel<MODE, MT, NB, 1>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+}
+cudaError_t allow_small_smem()
+{
+    cudaError_t e[] = {allow_small<SM_LAGRANGE, 1, 1>(), allow_small<SM_LAGRANGE, 2, 2>(), allow_small<SM_LAGRANGE, 3, 3>(),
+                       allow_small<SM_LAGRANGE, 4, 4>(), allow_small<SM_ONE, 1, 1>(), allow_small<SM_ONE, 1, 2>(),
+                       allow_small<SM_ONE, 1, 3>(), allow_small<SM_ONE, 1, 4>(), allow_small<SM_ONE, 2, 1>(),
+                       allow_small<SM_ONE, 2, 2>(), allow_small<SM_ONE, 2, 3>(), allow_small<SM_ONE, 2, 4>(),
+                       allow_small<SM_ONE, 3, 1>(), allow_small<SM_ONE, 3, 2>(), allow_small<SM_ONE, 3, 3>(),
+                       allow_small<SM_ONE, 3, 4>(), allow_small<SM_ONE, 4, 1>(), allow_small<SM_ONE, 4, 2>(),
+                       allow_small<SM_ONE, 4, 3>(), allow_small<SM_ONE, 4, 4>()};
+    for (cudaError_t x : e)
+        if (x != cudaSuccess) return x;
+    const void *k[] = {(const void *)small_proj_kernel<1>, (const void *)small_proj_kernel<2>,
+                       (const void *)small_proj_kernel<3>, (const void *)small_proj_kernel<4>};
+    for (const void *x : k) {
+        const cudaError_t r = cudaFuncSetAttribute(x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmProjSmem);
+        if (r != cudaSuccess) return r;
+    }
+    return cudaSuccess;
+}
+
+constexpr int kSmMaxBlocks = 64;  // tickets; more blocks take the general product
+
+// Plain products A'WB (a.A, a.B, a.m, a.n, a.C, a.ldc set) of `problems`
+// problems in blocks of up to 32 x 32; false in *done where they have too many blocks
+int small_products(cpsd_gpu_ctx *c, SmallArgs a, int problems, bool *done)
+{
+    const int m = std::max(a.m[0], a.m[1]), n = std::max(a.n[0], a.n[1]);
+    const int mt = (int)std::min<long>(4, cdiv(m, 8)), nt = (int)std::min<long>(4, cdiv(n, 8));
+    const long blocks = cdiv(m, 8 * mt) * cdiv(n, 8 * nt);
+    *done = blocks * problems <= kSmMaxBlocks;
+    if (!*done) return CPSD_OK;
+    a.K = 2 * c->npw_pad;
+    a.ld = 2L * c->npw_pad;
+    a.w = c->w;
+    a.part = c->gws;
+    a.ticket = c->ticket;
+    a.nblk = (int)cdiv(n, 8 * nt);
+    a.splits = small_splits(a.K, (int)blocks * problems);
+    const int bl = (int)blocks;
+    switch (4 * (mt - 1) + nt - 1) {
+#define CPSD_SMALL(M, N) \
+    case 4 * (M - 1) + N - 1: return launch_small<SM_ONE, M, N>(c, a, problems, bl, false);
+        CPSD_SMALL(1, 1) CPSD_SMALL(1, 2) CPSD_SMALL(1, 3) CPSD_SMALL(1, 4)
+        CPSD_SMALL(2, 1) CPSD_SMALL(2, 2) CPSD_SMALL(2, 3) CPSD_SMALL(2, 4)
+        CPSD_SMALL(3, 1) CPSD_SMALL(3, 2) CPSD_SMALL(3, 3) CPSD_SMALL(3, 4)
+        CPSD_SMALL(4, 1) CPSD_SMALL(4, 2) CPSD_SMALL(4, 3) CPSD_SMALL(4, 4)
+#undef CPSD_SMALL
+    default: return CPSD_ERR_ARG;
+    }
+}
+
+// Small cells' projector products on the 8 x 8 tile kernels: from K / 8 = 432 on
+// (64^3 / 16 bands / 32 projectors, 624: ten steps 758 -> 751 us; 12 uneven
+// cells 8.39 -> 7.54 ms; one band at 32^3, 2736: 154 -> 150 us).  On shorter
+// rows the four launches of the 64 x 64 tiles are as fast (24^3, 8 bands, 213:
+// 233 us, 238 here).
+bool small_projectors(const cpsd_gpu_ctx *c) { return c->nproj > 0 && small_cell(c) && 2L * c->npw_pad / 8 >= 432; }
+
+// Projector coefficients beta of the bands [lo, lo + nbl) (their orbitals in
+// c1l) and, with coef, the back-projection's coefficients (cpsd.c:287-289)
+int small_projector_products(cpsd_gpu_ctx *c, const cx<double> *c1l, int lo, int nbl, bool coef, bool *done)
+{
+    SmallArgs a{};
+    a.m[0] = c->nproj;
+    a.n[0] = nbl;
+    a.A[0] = (const double *)c->proj;
+    a.B[0] = (const double *)c1l;
+    a.C[0] = c->beta + lo;
+    a.ldc = c->nb;
+    if (coef) {
+        a.norm = c->vnlnrm_p;
+        a.scal2 = c->scal2;
+        a.coefT = c->coefT + (long)lo * c->nproj;
+        a.ldt = c->nproj;
+        a.coefP = c->move ? c->coefP + lo : nullptr;
+        a.ldp = c->nb;
+    }
+    return small_products(c, a, 1, done);
+}
+
+// out_j = sum_l mat[j * ldm + l] in_l, j < nj (small.cuh); *done false where
+// the matrix rows do not fit shared memory
+int small_projection(cpsd_gpu_ctx *c, int nj, int L, const double *mat, long ldm, const double *in, double *out, bool *done)
+{
+    SmallProjArgs a{2 * c->npw_pad, L, nj, 2L * c->npw_pad, ldm, mat, in, out};
+    const int mt = (int)std::min<long>(4, cdiv(nj, 8));
+    const size_t smem = sizeof(double) * 8 * mt * (size_t)small_proj_ld(L);
+    *done = smem <= kSmProjSmem;
+    if (!*done) return CPSD_OK;
+    const dim3 grid((unsigned)std::min<long>(2L * c->sms, cdiv(a.K / 16, kSmWarps)), (unsigned)cdiv(nj, 8 * mt));
+    switch (mt) {
+    case 1: launch(small_proj_kernel<1>, grid, kSmThreads, smem, c->cs, false, a); break;
+    case 2: launch(small_proj_kernel<2>, grid, kSmThreads, smem, c->cs, false, a); break;
+    case 3: launch(small_proj_kernel<3>, grid, kSmThreads, smem, c->cs, false, a); break;
+    default: launch(small_proj_kernel<4>, grid, kSmThreads, smem, c->cs, false, a); break;
+    }
+    c->nlaunch += 1;
+    return CPSD_OK;
 }
 
 // C_ms[i][j] = <A_i|B_j> over the bands of each spin (Gamma-point weights);
@@ -1003,9 +1139,19 @@ int small_overlaps(cpsd_gpu_ctx *c, SmallArgs a, const double *A, const double *
 int band_products(cpsd_gpu_ctx *c, const double *A, const double *B, double *const *C, int which = 0, bool upper = false)
 {
     if (small_cell(c)) {
-        SmallArgs a{};
-        for (int ms = 0; ms < c->ispin; ++ms) a.C[ms] = C[ms];
-        return small_overlaps<SM_ONE>(c, a, A, B);
+        for (int ms = 0; ms < c->ispin; ++ms) {  // (C's rows are the spin's own band count apart)
+            SmallArgs a{};
+            a.m[0] = a.n[0] = ms ? c->ne1 : c->ne0;
+            const long off = (long)(ms ? c->ne0 : 0) * 2L * c->npw_pad;
+            a.A[0] = A + off;
+            a.B[0] = B + off;
+            a.C[0] = C[ms];
+            a.ldc = a.m[0];
+            bool done = true;
+            const int rc = a.m[0] > 0 ? small_products(c, a, 1, &done) : CPSD_OK;
+            if (rc) return rc;
+        }
+        return CPSD_OK;
     }
     const long ldr = 2L * c->npw_pad;
     for (int ms = 0; ms < c->ispin; ++ms) {
@@ -1110,6 +1256,27 @@ int issue_knl(cpsd_gpu_ctx *c, cudaStream_t side, const cx<double> *c1, cx<doubl
     const cx<double> *c1l = c1 + (long)lo * c->ldc;
     cx<double> *c2l = c2 + (long)lo * c->ldc;
     c->cs = side;
+    if (small_projectors(c) && nbl > 0) {
+        // coefficients beta and coef in one launch, then the back-projection
+        bool tn = true, nn = true;
+        int rc = small_projector_products(c, c1l, lo, nbl, true, &tn);
+        if (!rc && tn)
+            rc = small_projection(c, nbl, c->nproj, c->coefT + (long)lo * c->nproj, c->nproj, (const double *)c->proj,
+                                  (double *)c2l, &nn);
+        if (!rc && tn && !nn)
+            gemm_nn(c, nbl, K, c->nproj, 1.0, c->coefT + (long)lo * c->nproj, c->nproj, (const double *)c->proj, ldr, 0.0,
+                    (double *)c2l, ldr, TN_PROJECTOR);
+        if (!rc && tn && c->move) {
+            bool fn = true;
+            rc = small_projection(c, c->nproj, c->nb, c->coefP, c->nb, (const double *)c1, (double *)c->Ynl, &fn);
+            force_nonlocal_kernel<<<c->nproj, 256, 0, side>>>(c->npw, c->ldc, c->w, c->Gv, c->proj, c->Ynl, c->fnl);
+            c->nlaunch += 1;
+        }
+        if (rc || tn) {
+            c->cs = s;
+            return rc;
+        }
+    }
     if (c->nproj > 0) {
         int rc = gemm_tn(c, c->nproj, nbl, K, (const double *)c->proj, ldr, (const double *)c1l, ldr, c->w, 1.0,
                          0.0, c->beta + lo, c->nb, TN_PROJECTOR);
@@ -1358,9 +1525,7 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
     la.fail = c->flags;
     const double *lmds[2] = {c->lmd, c->lmd + ne02};
     if (small_cell(c)) {  // overlaps and solver in one launch
-        SmallArgs a{};
-        a.lag = la;
-        int rc = small_overlaps<SM_LAGRANGE>(c, a, (const double *)c2, (const double *)c1, chain && !c->mlp);
+        int rc = small_overlaps(c, la, (const double *)c2, (const double *)c1, chain && !c->mlp);
         if (rc) return rc;
         mark(c, 10);
         mark(c, 11);
@@ -2500,7 +2665,7 @@ int cpsd_gpu_create(const cpsd_gpu_params *p, const int *masker1, cpsd_gpu_ctx *
     CK(ar.alloc(&c->red, 2 * kLagClusterMax));
     CK(ar.alloc(&c->Edev, 16));
     CK(ar.alloc(&c->flags, 4));
-    CK(ar.alloc(&c->ticket, 1));
+    CK(ar.alloc(&c->ticket, kSmMaxBlocks));
     c->gemm_splits_cap = 512;
     // split-K partials: at least 32 MB, and room for one split per SM of the
     // three overlaps of the largest spin
@@ -2536,23 +2701,7 @@ int cpsd_gpu_create(const cpsd_gpu_params *p, const int *masker1, cpsd_gpu_ctx *
     CK(ar.alloc(&c->py, (size_t)nb * kShells));
     CK(allow_dm_smem());
     if (small_cell(c.get())) {
-        auto allow = [&](auto one, auto lag, size_t so, size_t sl) {
-            cudaError_t e = cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)so);
-            return e != cudaSuccess ? e : cudaFuncSetAttribute(lag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sl);
-        };
-        cudaError_t e = cudaSuccess;
-        const int top = kLagSmallMax;  // the attribute is the kernel's, shared by every context
-        switch (cdiv(c->ne0, 8)) {
-        case 1: e = allow(small_overlap_kernel<SM_ONE, 1>, small_overlap_kernel<SM_LAGRANGE, 1>,
-                          small_smem_bytes<SM_ONE, 1>(top), small_smem_bytes<SM_LAGRANGE, 1>(top)); break;
-        case 2: e = allow(small_overlap_kernel<SM_ONE, 2>, small_overlap_kernel<SM_LAGRANGE, 2>,
-                          small_smem_bytes<SM_ONE, 2>(top), small_smem_bytes<SM_LAGRANGE, 2>(top)); break;
-        case 3: e = allow(small_overlap_kernel<SM_ONE, 3>, small_overlap_kernel<SM_LAGRANGE, 3>,
-                          small_smem_bytes<SM_ONE, 3>(top), small_smem_bytes<SM_LAGRANGE, 3>(top)); break;
-        default: e = allow(small_overlap_kernel<SM_ONE, 4>, small_overlap_kernel<SM_LAGRANGE, 4>,
-                           small_smem_bytes<SM_ONE, 4>(top), small_smem_bytes<SM_LAGRANGE, 4>(top)); break;
-        }
-        CK(e);
+        CK(allow_small_smem());
     }
     else {
         // 16-CTA clusters where the device can schedule them, else the portable 8
@@ -3358,7 +3507,12 @@ int cpsd_gpu_bp_finish(cpsd_gpu_ctx *c, int inner, double *E, double *deltae, do
     CK(cudaMemcpyAsync(c->Edev, E, sizeof(double), cudaMemcpyHostToDevice, s));
     // the projector coefficients of every band (the steps formed only this
     // rank's columns); c1 is the last step's orbitals of all bands
-    if (c->nproj > 0) {
+    bool done = false;
+    if (small_projectors(c)) {
+        int rc = small_projector_products(c, c->cbuf[c->cur ^ 1], 0, c->nb, false, &done);
+        if (rc) return rc;
+    }
+    if (c->nproj > 0 && !done) {
         const long ldr = 2L * c->npw_pad;
         int rc = gemm_tn(c, c->nproj, c->nb, 2 * c->npw_pad, (const double *)c->proj, ldr,
                          (const double *)c->cbuf[c->cur ^ 1], ldr, c->w, 1.0, 0.0, c->beta, c->nb, TN_PROJECTOR);

@@ -16,34 +16,48 @@
 
 constexpr int kSmThreads = 256, kSmWarps = kSmThreads / 32, kSmCluster = 8;
 constexpr int kSmMaxClusters = 18;  // 144 CTAs: one per SM
+// Rows of up to this many steps of 8 reals are split over at most 18 CTAs whose
+// sums the last one adds: the cluster's two barriers cost more there than they
+// save (six steps a warp; 64^3, 16 bands, ten steps: 765 us with clusters, 751
+// without).
+constexpr int kSmNoClusterSteps = kSmMaxClusters * kSmWarps * 6;
 
 // products of one launch: the three overlaps (C2'WC2 and C1'WC1 by their upper
-// tiles, C2'WC1 whole), or one plain product A'WB
+// tiles, C2'WC1 whole; MT tiles of 8 bands), or plain products A'WB in blocks
+// of up to MT x NB tiles
 enum { SM_LAGRANGE = 0, SM_ONE = 1 };
-template <int MODE, int MT>
+template <int MODE, int MT, int NB>
 constexpr int sm_tiles()
 {
-    return MODE == SM_LAGRANGE ? MT * (MT + 1) + MT * MT : MT * MT;
+    return MODE == SM_LAGRANGE ? MT * (MT + 1) + MT * MT : MT * NB;
 }
 
 struct SmallArgs {
-    int K, splits;               // reals per row; CTAs along k (a multiple of kSmCluster)
+    int K, splits;               // reals per row; CTAs along k (a multiple of the cluster size)
     long ld;                     // reals between rows
-    int m[2];                    // bands per spin (spins = gridDim.y)
+    int m[2], n[2];              // rows of A and of B, per spin or problem (gridDim.y)
     const double *A[2], *B[2];   // LAGRANGE: C2 and C1 of a spin; ONE: the two operands
     const double *w;             // weight per pair of reals
-    double *part;                // [spin][cluster][tiles * 64]
-    unsigned *ticket;            // zero before the launch, zero after it
-    double *C[2];                // ONE: C[i * m + j]
+    double *part;                // [block][cluster][tiles * 64]
+    unsigned *ticket;            // one per block (LAGRANGE: one), zero before the launch and after it
+    double *C[2];                // ONE: C[i * ldc + j]
+    long ldc;
+    int nblk;                    // ONE: gridDim.z = blocks of 8 MT rows of A x nblk blocks of 8 NB rows of B
+    // ONE, projector coefficients: coefT[j][i] = -C scal2 / norm[i] (cpsd.c:289;
+    // and coefP[i][j], for the nonlocal force) beside C; null otherwise
+    const double *norm;
+    double *coefT, *coefP;
+    long ldt, ldp;
+    double scal2;
     LagArgs lag;                 // LAGRANGE
 };
 
-template <int MODE, int MT>
+template <int MODE, int MT, int NB>
 size_t small_smem_bytes(int ne0)
 {
-    const size_t red = (size_t)(kSmWarps / 2) * sm_tiles<MODE, MT>() * 64;
+    const size_t red = (size_t)(kSmWarps / 2) * sm_tiles<MODE, MT, NB>() * 64;
     constexpr int mp = 8 * MT, ld = (mp % 16 == 8) ? mp : mp + 8;
-    const size_t solve = MODE == SM_LAGRANGE ? (size_t)sm_tiles<MODE, MT>() * 64 + 3 * mp * ld + (size_t)ne0 * ne0 : 0;
+    const size_t solve = MODE == SM_LAGRANGE ? (size_t)sm_tiles<MODE, MT, NB>() * 64 + 3 * mp * ld + (size_t)ne0 * ne0 : 0;
     return sizeof(double) * (red > solve ? red : solve);
 }
 
@@ -232,51 +246,57 @@ CPSD_D void small_lagrange(const LagArgs &a, int ms, int m, const double *S, dou
     }
 }
 
-template <int MODE, int MT>
+// CL: CTAs of a cluster (kSmCluster, or 1: no cluster)
+template <int MODE, int MT, int NB, int CL>
 __global__ void __launch_bounds__(kSmThreads, 1) small_overlap_kernel(const __grid_constant__ SmallArgs a)
 {
-    constexpr int NT = sm_tiles<MODE, MT>(), NTRI = MT * (MT + 1) / 2, E = NT * 64;
-    cg::cluster_group cl = cg::this_cluster();
+    static_assert(MODE == SM_ONE || MT == NB, "square");
+    constexpr int NT = sm_tiles<MODE, MT, NB>(), NTRI = MT * (MT + 1) / 2, E = NT * 64;
     extern __shared__ __align__(16) double sm_raw[];
     __shared__ unsigned slot[kSmWarps][4];
     __shared__ int last;
     chain_wait();
     chain_start();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = lane >> 2, q = lane & 3;
-    const int ms = blockIdx.y, m = a.m[ms];
-    const double *__restrict__ A = a.A[ms], *__restrict__ B = a.B[ms];
+    const int ms = blockIdx.y;
+    const int ia = MODE == SM_ONE ? (int)blockIdx.z / a.nblk * (8 * MT) : 0;  // first rows of this block
+    const int ib = MODE == SM_ONE ? (int)blockIdx.z % a.nblk * (8 * NB) : 0;
+    const int ma = a.m[ms] - ia, mb = (MODE == SM_ONE ? a.n[ms] : a.m[ms]) - ib;
+    const double *__restrict__ A = a.A[ms] + ia * a.ld, *__restrict__ B = a.B[ms] + ib * a.ld;
     // this warp's slice of k, in steps of 8 reals (a lane's 16 bytes of a row
     // feed two MMA k-steps: reals 2q of the step, then 2q + 1)
     const int n8 = a.K / 8, nw = a.splits * kSmWarps, wid = blockIdx.x * kSmWarps + warp;
     const int per = (n8 + nw - 1) / nw, s0 = min(n8, wid * per), s1 = min(n8, s0 + per);
     double acc[NT][2] = {};
-    const double2 *pa[MT], *pb[MT];
-    bool ok[MT];
+    const double2 *pa[MT], *pb[NB];
+    bool oka[MT], okb[NB];
 #pragma unroll
     for (int i = 0; i < MT; ++i) {
-        ok[i] = 8 * i + r < m;
-        pa[i] = reinterpret_cast<const double2 *>(A + (long)(ok[i] ? 8 * i + r : 0) * a.ld + 2 * q);
-        pb[i] = reinterpret_cast<const double2 *>(B + (long)(ok[i] ? 8 * i + r : 0) * a.ld + 2 * q);
+        oka[i] = 8 * i + r < ma;
+        pa[i] = reinterpret_cast<const double2 *>(A + (long)(oka[i] ? 8 * i + r : 0) * a.ld + 2 * q);
     }
-    double2 na[MT], nb[MT];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+        okb[i] = 8 * i + r < mb;
+        pb[i] = reinterpret_cast<const double2 *>(B + (long)(okb[i] ? 8 * i + r : 0) * a.ld + 2 * q);
+    }
+    double2 na[MT], nb[NB];
     double nw8 = 0.0;
     auto fetch = [&](int s) {
         nw8 = a.w[4 * s + q];
 #pragma unroll
-        for (int i = 0; i < MT; ++i) {
-            na[i] = ok[i] ? pa[i][4 * s] : make_double2(0.0, 0.0);
-            nb[i] = ok[i] ? pb[i][4 * s] : make_double2(0.0, 0.0);
-        }
+        for (int i = 0; i < MT; ++i) na[i] = oka[i] ? pa[i][4 * s] : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int i = 0; i < NB; ++i) nb[i] = okb[i] ? pb[i][4 * s] : make_double2(0.0, 0.0);
     };
     if (s0 < s1) fetch(s0);
     for (int s = s0; s < s1; ++s) {
-        double2 xa[MT], xb[MT];
+        double2 xa[MT], xb[NB];
         const double ww = nw8;
 #pragma unroll
-        for (int i = 0; i < MT; ++i) {
-            xa[i] = na[i];
-            xb[i] = nb[i];
-        }
+        for (int i = 0; i < MT; ++i) xa[i] = na[i];
+#pragma unroll
+        for (int i = 0; i < NB; ++i) xb[i] = nb[i];
         if (s + 1 < s1) fetch(s + 1);
         int t = 0;
         if constexpr (MODE == SM_LAGRANGE) {
@@ -308,7 +328,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) small_overlap_kernel(const __gr
             for (int i = 0; i < MT; ++i) {
                 const double2 wa = make_double2(xa[i].x * ww, xa[i].y * ww);
 #pragma unroll
-                for (int j = 0; j < MT; ++j, ++t) {
+                for (int j = 0; j < NB; ++j, ++t) {
                     dmma(acc[t][0], acc[t][1], wa.x, xb[j].x);
                     dmma(acc[t][0], acc[t][1], wa.y, xb[j].y);
                 }
@@ -342,36 +362,44 @@ __global__ void __launch_bounds__(kSmThreads, 1) small_overlap_kernel(const __gr
             *reinterpret_cast<double2 *>(red + t * 64 + 2 * lane) = make_double2(acc[t][0], acc[t][1]);
     }
     // entry t * 64 + 8 r + 2 q + e: row r, column 2 q + e of tile t
-    cl.sync();
-    const int rank = (int)cl.block_rank(), ncl = a.splits / kSmCluster, cid = blockIdx.x / kSmCluster;
-    double *part = a.part + (size_t)ms * kSmMaxClusters * E;
-    {
-        const double *src[kSmCluster];
+    const int ncl = a.splits / CL, cid = blockIdx.x / CL;
+    const int blk = blockIdx.y * gridDim.z + blockIdx.z;
+    double *part = a.part + (size_t)blk * kSmMaxClusters * E;
+    if constexpr (CL > 1) {
+        cg::cluster_group cl = cg::this_cluster();
+        cl.sync();
+        const int rank = (int)cl.block_rank();
+        const double *src[CL];
 #pragma unroll
-        for (int c = 0; c < kSmCluster; ++c) src[c] = cl.map_shared_rank(red, c);
-        for (int e = rank * kSmThreads + tid; e < E; e += kSmCluster * kSmThreads) {
-            double v[kSmCluster], s = 0.0;
+        for (int c = 0; c < CL; ++c) src[c] = cl.map_shared_rank(red, c);
+        for (int e = rank * kSmThreads + tid; e < E; e += CL * kSmThreads) {
+            double v[CL], s = 0.0;
 #pragma unroll
-            for (int c = 0; c < kSmCluster; ++c) v[c] = src[c][e];
+            for (int c = 0; c < CL; ++c) v[c] = src[c][e];
 #pragma unroll
-            for (int c = 0; c < kSmCluster; ++c) s += v[c];
+            for (int c = 0; c < CL; ++c) s += v[c];
             part[(size_t)cid * E + e] = s;
         }
+        cl.sync();  // the peers have read this CTA's tiles
+    } else {
+        __syncthreads();
+        for (int e = tid; e < E; e += kSmThreads) part[(size_t)cid * E + e] = red[e];
     }
-    cl.sync();  // the peers have read this CTA's tiles
     __threadfence();
     __syncthreads();
     if (tid == 0) {
-        const unsigned total = gridDim.x * gridDim.y;
-        last = atomicAdd(a.ticket, 1u) == total - 1;
-        if (last) *a.ticket = 0;  // for the next launch
+        // the last CTA of a block (of the launch, for the solver)
+        const unsigned total = MODE == SM_ONE ? gridDim.x : gridDim.x * gridDim.y;
+        unsigned *tk = a.ticket + (MODE == SM_ONE ? blk : 0);
+        last = atomicAdd(tk, 1u) == total - 1;
+        if (last) *tk = 0;  // for the next launch
     }
     __syncthreads();
     if (!last) return;
     __threadfence();
-    for (int sp = 0; sp < (int)gridDim.y; ++sp) {
-        const int mm = a.m[sp];
-        const double *ps = a.part + (size_t)sp * kSmMaxClusters * E;
+    const int sp0 = MODE == SM_ONE ? ms : 0, sp1 = MODE == SM_ONE ? ms + 1 : (int)gridDim.y;
+    for (int sp = sp0; sp < sp1; ++sp) {
+        const double *ps = a.part + (size_t)(MODE == SM_ONE ? blk : sp) * kSmMaxClusters * E;
         double *S = sm_raw;
         for (int e = tid; e < E; e += kSmThreads) {
             double v[kSmMaxClusters], s = 0.0;
@@ -382,12 +410,20 @@ __global__ void __launch_bounds__(kSmThreads, 1) small_overlap_kernel(const __gr
             if constexpr (MODE == SM_LAGRANGE) {
                 S[e] = s;
             } else {
-                const int t = e / 64, i = 8 * (t / MT) + (e % 64) / 8, j = 8 * (t % MT) + e % 8;
-                if (i < mm && j < mm) a.C[sp][i * mm + j] = s;
+                const int t = e / 64, i = 8 * (t / NB) + (e % 64) / 8, j = 8 * (t % NB) + e % 8;
+                if (i < ma && j < mb) {
+                    a.C[sp][(long)(ia + i) * a.ldc + ib + j] = s;
+                    if (a.norm) {
+                        const double v = -s * a.scal2 / a.norm[ia + i];
+                        a.coefT[(long)(ib + j) * a.ldt + ia + i] = v;
+                        if (a.coefP) a.coefP[(long)(ia + i) * a.ldp + ib + j] = v;
+                    }
+                }
             }
         }
         if constexpr (MODE == SM_LAGRANGE) {
             __syncthreads();
+            const int mm = a.m[sp];
             if (mm > 0 && (MT > 1 || warp == 0)) small_lagrange<MT>(a.lag, sp, mm, S, sm_raw + E, slot);
             __syncthreads();
         }
@@ -451,6 +487,56 @@ __global__ void __launch_bounds__(kSmThreads) small_nn_kernel(const __grid_const
                 }
                 o[0] = make_double2(a.alpha * e0[0] + a.beta * v0.x, a.alpha * e1[0] + a.beta * v0.y);
                 o[1] = make_double2(a.alpha * e0[1] + a.beta * v1.x, a.alpha * e1[1] + a.beta * v1.y);
+            }
+        }
+    }
+}
+
+// out_j = sum_l mat[j * ldm + l] in_l for up to 8 MT rows
+// j per blockIdx.y and any number of l (the KB back-projection of a small cell:
+// l over the projectors).  As small_nn_kernel, with the matrix rows in shared
+// memory, LD = 4 mod 16 apart (a 16-lane phase then hits 16 banks).
+CPSD_HD int small_proj_ld(int L) { return (L + 7) / 8 * 8 + ((L + 7) / 8 % 2 ? 12 : 4); }
+struct SmallProjArgs {
+    int K, L, nj;
+    long ld, ldm;   // reals between the rows of in / out; of mat
+    const double *mat, *in;
+    double *out;
+};
+
+template <int MT>
+__global__ void __launch_bounds__(kSmThreads) small_proj_kernel(const __grid_constant__ SmallProjArgs a)
+{
+    extern __shared__ __align__(16) double sp_mat[];
+    const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
+    const int j0 = blockIdx.y * 8 * MT, LD = small_proj_ld(a.L), Lp = (a.L + 7) / 8 * 8;
+    for (int e = threadIdx.x; e < 8 * MT * Lp; e += kSmThreads) {
+        const int j = e / Lp, l = e % Lp;
+        sp_mat[j * LD + l] = (j0 + j < a.nj && l < a.L) ? a.mat[(long)(j0 + j) * a.ldm + l] : 0.0;
+    }
+    __syncthreads();
+    const int nblk = a.K / 16, nw = gridDim.x * kSmWarps;
+    for (int b = blockIdx.x * kSmWarps + (threadIdx.x >> 5); b < nblk; b += nw) {
+        double e0[MT][2] = {}, e1[MT][2] = {};
+        const double *src = a.in + 16 * b + 2 * r;
+#pragma unroll 4
+        for (int l0 = 0; l0 < Lp; l0 += 4) {
+            const int l = l0 + q;
+            const double2 x = l < a.L ? *reinterpret_cast<const double2 *>(src + (long)l * a.ld) : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int j = 0; j < MT; ++j) {
+                const double c = sp_mat[(8 * j + r) * LD + l];
+                dmma(e0[j][0], e0[j][1], c, x.x);
+                dmma(e1[j][0], e1[j][1], c, x.y);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < MT; ++j) {
+            const int jj = j0 + 8 * j + r;
+            if (jj < a.nj) {
+                double2 *o = reinterpret_cast<double2 *>(a.out + (long)jj * a.ld + 16 * b + 4 * q);
+                o[0] = make_double2(e0[j][0], e1[j][0]);
+                o[1] = make_double2(e0[j][1], e1[j][1]);
             }
         }
     }
