@@ -52,6 +52,7 @@ cudaError_t &last_cuda_error()
 
 inline long cdiv(long a, long b) { return (a + b - 1) / b; }
 
+constexpr int kEnergyNlBlocks = 64;  // blocks of the nonlocal energy's sum
 constexpr int kTuneMaxCtas = 8;  // largest split-K target (CTAs per SM) a tuning may set
 // trust region of the guarded learned step (cpsd_gpu_run_guarded): the bound
 // on log K shrinks after a rejected block and grows after an accepted one
@@ -711,7 +712,7 @@ struct cpsd_gpu_ctx {
     std::vector<char> tables_last;  // the staged bytes of the last upload (a repeat is not sent again)
     Pinned dstage;  // the density (ispin * n^3) on its way to the padded host layout
     int pblocks = 0, bblocks = 0, gblocks = 0;
-    double *ppart = nullptr, *bpart = nullptr, *gpart = nullptr;
+    double *ppart = nullptr, *bpart = nullptr, *gpart = nullptr, *npart = nullptr;
 };
 
 namespace {
@@ -1724,17 +1725,54 @@ int energies(cpsd_gpu_ctx *c, int inner)
     if (rc) return rc;
     fa.Mh[0] = Mh[0];
     fa.Mh[1] = Mh[1];
-    packed_terms_kernel<<<c->pblocks, 256, 0, s>>>(c->npw, c->w, c->sfac, c->vg, c->dng, c->vc, c->vall,
-                                                   c->ppart); c->nlaunch += 1;
-    band_terms_kernel<<<dim3(c->bblocks, c->nb), 256, 0, s>>>(c->npw, c->ldc, c->w, c->tg, c1, c2, c->bpart); c->nlaunch += 1;
-    grid_terms_kernel<<<c->gblocks, 256, 0, s>>>(c->n3, c->ispin, c->dn, c->xce, c->xcp, c->gpart); c->nlaunch += 1;
+    EnergyArgs ea{};
+    ea.pblocks = c->pblocks;
+    ea.bblocks = c->bblocks;
+    ea.gblocks = c->gblocks;
+    ea.eblocks = std::max(0, c->nion - 1);
+    ea.nblocks = c->nproj > 0 ? (int)std::min<long>(kEnergyNlBlocks, cdiv((long)c->nproj * c->nb, 256)) : 0;
+    ea.npw = c->npw;
+    ea.nb = c->nb;
+    ea.ispin = c->ispin;
+    ea.nion = c->nion;
+    ea.nsh = c->nsh;
+    ea.nproj = c->nproj;
+    ea.ldc = c->ldc;
+    ea.n3 = c->n3;
+    ea.w = c->w;
+    ea.tg = c->tg;
+    ea.vg = c->vg;
+    ea.vc = c->vc;
+    ea.dn = c->dn;
+    ea.xce = c->xce;
+    ea.xcp = c->xcp;
+    ea.r1 = c->r1;
+    ea.rcell = c->rcell;
+    ea.zv = c->zv;
+    ea.beta = c->beta;
+    ea.vnlnrm_p = c->vnlnrm_p;
+    ea.katm = c->katm;
+    ea.s = c->sfac;
+    ea.dng = c->dng;
+    ea.vall = c->vall;
+    ea.c1 = c1;
+    ea.c2 = c2;
+    ea.rcut = c->prm.rcut;
+    ea.scal2 = c->scal2;
+    ea.ppart = c->ppart;
+    ea.bpart = c->bpart;
+    ea.gpart = c->gpart;
+    ea.epart = c->epart;
+    ea.npart = c->npart;
+    energy_terms_kernel<<<ea.pblocks + ea.bblocks * ea.nb + ea.gblocks + ea.eblocks + ea.nblocks, 256, 0, s>>>(ea);
+    c->nlaunch += 1;
     fa.ispin = c->ispin;
     fa.ne0 = c->ne0;
     fa.ne1 = c->ne1;
     fa.nion = c->nion;
-    fa.nsh = c->nsh;
-    fa.nproj = c->nproj;
     fa.nb = c->nb;
+    fa.nblocks = ea.nblocks;
+    fa.npart = c->npart;
     fa.inner = inner;
     fa.pblocks = c->pblocks;
     fa.bblocks = c->bblocks;
@@ -1743,19 +1781,11 @@ int energies(cpsd_gpu_ctx *c, int inner)
     fa.bpart = c->bpart;
     fa.gpart = c->gpart;
     fa.hml = c->hml;
-    fa.beta = c->beta;
-    fa.vnlnrm_p = c->vnlnrm_p;
-    if (c->nion > 1) {
-        ewald_real_kernel<<<c->nion - 1, 256, 0, s>>>(c->nion, c->nsh, c->r1, c->rcell, c->zv, c->katm,
-                                                      c->prm.rcut, c->epart);
-        c->nlaunch += 1;
-    }
     fa.ewald_part = c->epart;
     fa.scal2 = c->scal2;
     fa.omega = c->prm.omega;
     fa.dv = c->dv;
     fa.cewald = c->prm.cewald;
-    fa.rcut = c->prm.rcut;
     fa.dt = c->prm.dt;
     fa.dte = c->dte;
     fa.E = c->Edev;
@@ -2677,6 +2707,7 @@ int cpsd_gpu_create(const cpsd_gpu_params *p, const int *masker1, cpsd_gpu_ctx *
     CK(ar.alloc(&c->ppart, 3 * c->pblocks));
     CK(ar.alloc(&c->bpart, (size_t)2 * nb * c->bblocks));
     CK(ar.alloc(&c->gpart, 2 * c->gblocks));
+    CK(ar.alloc(&c->npart, kEnergyNlBlocks));
     CK(cudaMallocHost((void **)&c->hstage.p, sizeof(cx<double>) * 2 * nb * c->ldc));
     {
         // every slice cpsd_gpu_set_tables packs, each rounded up to 16 bytes

@@ -1242,127 +1242,137 @@ __global__ void __launch_bounds__(kLagThreads) lagrange_tile_kernel(LagArgs a)
 }
 
 // ------------------------------------------------------------ energies
-// per-block partial sums over packed points of the three single-field terms
-// (cpsd.c:520-526 k-space Ewald, :548-554 Hartree, :590 local)
-__global__ void packed_terms_kernel(int npw, const double *__restrict__ w, const cx<double> *__restrict__ s,
-                                    const double *__restrict__ vg, const cx<double> *__restrict__ dng,
-                                    const double *__restrict__ vc, const cx<double> *__restrict__ vall,
-                                    double *part)
-{
-    __shared__ double sh[32];
-    double e0 = 0, e1 = 0, e2 = 0;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npw; p += gridDim.x * blockDim.x) {
-        const double ww = w[p];
-        const cx<double> sv = s[p], d = dng[p], va = vall[p];
-        e0 += ww * (sv.x * sv.x + sv.y * sv.y) * vg[p];
-        e1 += ww * (d.x * d.x + d.y * d.y) * vc[p];
-        e2 += ww * (va.x * d.x + va.y * d.y);
-    }
-    double r0 = block_sum<256>(e0, sh);
-    double r1 = block_sum<256>(e1, sh);
-    double r2 = block_sum<256>(e2, sh);
-    if (threadIdx.x == 0) {
-        part[blockIdx.x] = r0;
-        part[gridDim.x + blockIdx.x] = r1;
-        part[2 * gridDim.x + blockIdx.x] = r2;
-    }
-}
+// Every partial sum of the energies in one launch (five before; they are
+// independent and each a few microseconds): block ranges in the order of
+// EnergyArgs' counts, every block a fixed-order sum.
+struct EnergyArgs {
+    int pblocks, bblocks, gblocks, eblocks, nblocks;  // packed, per band, grid, Ewald (ions - 1), nonlocal
+    int npw, nb, ispin, nion, nsh, nproj;
+    long ldc, n3;
+    const double *w, *tg, *vg, *vc, *dn, *xce, *xcp, *r1, *rcell, *zv, *beta, *vnlnrm_p;
+    const int *katm;
+    const cx<double> *s, *dng, *vall, *c1, *c2;
+    double rcut, scal2;
+    double *ppart;  // [3][pblocks]: k-space Ewald, Hartree, local (cpsd.c:520-526, 548-554, 590)
+    double *bpart;  // [2][nb][bblocks]: eke_b (cpsd.c:574-586), dc_b (:650-659)
+    double *gpart;  // [2][gblocks]: exc, pxc (cpsd.c:557-570)
+    double *epart;  // [nion - 1]: real-space Ewald of the pairs (ii, jj > ii)
+    double *npart;  // [nblocks]: nonlocal energy of the last step's projections (cpsd.c:593-634)
+};
 
-// per band: eke_b = sum w tg |c1|^2 (cpsd.c:574-586), dc_b = sum w |c2-c1|^2 (:650-659)
-__global__ void band_terms_kernel(int npw, long ldc, const double *__restrict__ w,
-                                  const double *__restrict__ tg, const cx<double> *__restrict__ c1,
-                                  const cx<double> *__restrict__ c2, double *part /* [2][nb][blocks] */)
+__global__ void __launch_bounds__(256) energy_terms_kernel(const __grid_constant__ EnergyArgs a)
 {
     __shared__ double sh[32];
-    const int b = blockIdx.y;
-    const cx<double> *a = c1 + (long)b * ldc, *c = c2 + (long)b * ldc;
-    double ek = 0, dc = 0;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npw; p += gridDim.x * blockDim.x) {
-        const double ww = w[p];
-        const cx<double> x = a[p], y = c[p];
-        ek += ww * tg[p] * (x.x * x.x + x.y * x.y);
-        const double dx = y.x - x.x, dy = y.y - x.y;
-        dc += ww * (dx * dx + dy * dy);
-    }
-    double r0 = block_sum<256>(ek, sh);
-    double r1 = block_sum<256>(dc, sh);
-    if (threadIdx.x == 0) {
-        part[(long)b * gridDim.x + blockIdx.x] = r0;
-        part[((long)gridDim.y + b) * gridDim.x + blockIdx.x] = r1;
-    }
-}
-
-// exc, pxc partial sums over the real grid (cpsd.c:557-570)
-__global__ void grid_terms_kernel(long n3, int ispin, const double *__restrict__ dn,
-                                  const double *__restrict__ xce, const double *__restrict__ xcp,
-                                  double *part)
-{
-    __shared__ double sh[32];
-    double ex = 0, px = 0;
-    for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n3; r += (long)gridDim.x * blockDim.x) {
-        const double d0 = dn[r];
-        ex += d0 * xce[r];
-        px += d0 * xcp[r];
-        if (ispin == 2) {
-            const double d1 = dn[n3 + r];
-            ex += d1 * xce[r];
-            px += d1 * xcp[n3 + r];
+    const int tid = threadIdx.x;
+    int blk = blockIdx.x;
+    if (blk < a.pblocks) {
+        double e0 = 0, e1 = 0, e2 = 0;
+        for (int p = blk * 256 + tid; p < a.npw; p += a.pblocks * 256) {
+            const double ww = a.w[p];
+            const cx<double> sv = a.s[p], d = a.dng[p], va = a.vall[p];
+            e0 += ww * (sv.x * sv.x + sv.y * sv.y) * a.vg[p];
+            e1 += ww * (d.x * d.x + d.y * d.y) * a.vc[p];
+            e2 += ww * (va.x * d.x + va.y * d.y);
         }
+        const double r0 = block_sum<256>(e0, sh), r1 = block_sum<256>(e1, sh), r2 = block_sum<256>(e2, sh);
+        if (tid == 0) {
+            a.ppart[blk] = r0;
+            a.ppart[a.pblocks + blk] = r1;
+            a.ppart[2 * a.pblocks + blk] = r2;
+        }
+        return;
     }
-    double r0 = block_sum<256>(ex, sh);
-    double r1 = block_sum<256>(px, sh);
-    if (threadIdx.x == 0) {
-        part[blockIdx.x] = r0;
-        part[gridDim.x + blockIdx.x] = r1;
+    blk -= a.pblocks;
+    if (blk < a.bblocks * a.nb) {
+        const int b = blk / a.bblocks, x = blk % a.bblocks;
+        const cx<double> *c1 = a.c1 + (long)b * a.ldc, *c2 = a.c2 + (long)b * a.ldc;
+        double ek = 0, dc = 0;
+        for (int p = x * 256 + tid; p < a.npw; p += a.bblocks * 256) {
+            const double ww = a.w[p];
+            const cx<double> u = c1[p], v = c2[p];
+            ek += ww * a.tg[p] * (u.x * u.x + u.y * u.y);
+            const double dx = v.x - u.x, dy = v.y - u.y;
+            dc += ww * (dx * dx + dy * dy);
+        }
+        const double r0 = block_sum<256>(ek, sh), r1 = block_sum<256>(dc, sh);
+        if (tid == 0) {
+            a.bpart[(long)b * a.bblocks + x] = r0;
+            a.bpart[((long)a.nb + b) * a.bblocks + x] = r1;
+        }
+        return;
+    }
+    blk -= a.bblocks * a.nb;
+    if (blk < a.gblocks) {
+        double ex = 0, px = 0;
+        for (long r = (long)blk * 256 + tid; r < a.n3; r += (long)a.gblocks * 256) {
+            const double d0 = a.dn[r], e = a.xce[r];
+            ex += d0 * e;
+            px += d0 * a.xcp[r];
+            if (a.ispin == 2) {
+                const double d1 = a.dn[a.n3 + r];
+                ex += d1 * e;
+                px += d1 * a.xcp[a.n3 + r];
+            }
+        }
+        const double r0 = block_sum<256>(ex, sh), r1 = block_sum<256>(px, sh);
+        if (tid == 0) {
+            a.gpart[blk] = r0;
+            a.gpart[a.gblocks + blk] = r1;
+        }
+        return;
+    }
+    blk -= a.gblocks;
+    if (blk < a.eblocks) {
+        // real-space Ewald, cpsd.c:527-545 (A&S 7.1.28 erfc, cpsd.c:11-17): the
+        // pairs (ii, jj > ii) over the nsh image cells, a (pair, image) per thread
+        const double B1 = 0.0705230784, B2 = 0.0422820123, B3 = 0.0092705272;
+        const double B4 = 0.0001520143, B5 = 0.0002765672, B6 = 0.0000430638;
+        const int ii = blk;
+        const long cnt = (long)(a.nion - 1 - ii) * a.nsh;
+        double ew = 0.0;
+        for (long e = tid; e < cnt; e += 256) {
+            const int jj = ii + 1 + (int)(e / a.nsh);
+            const int l = (int)(e % a.nsh);
+            const double dx = a.r1[3 * ii] - a.r1[3 * jj];
+            const double dy = a.r1[1 + 3 * ii] - a.r1[1 + 3 * jj];
+            const double dz = a.r1[2 + 3 * ii] - a.r1[2 + 3 * jj];
+            const double zz = a.zv[a.katm[ii]] * a.zv[a.katm[jj]];
+            const double x = a.rcell[l] + dx, y = a.rcell[l + a.nsh] + dy, z = a.rcell[l + 2 * a.nsh] + dz;
+            const double r = sqrt(x * x + y * y + z * z);
+            const double w = r / a.rcut;
+            const double aa = (1.0 + w * (B1 + w * (B2 + w * (B3 + w * (B4 + w * (B5 + w * B6))))));
+            const double erfc = 1.0 / (aa * aa * aa * aa);
+            ew += zz * (erfc * erfc * erfc * erfc) / r;
+        }
+        const double t = block_sum<256>(ew, sh);
+        if (tid == 0) a.epart[ii] = t;
+        return;
+    }
+    blk -= a.eblocks;
+    {
+        double en = 0.0;
+        const long cnt = (long)a.nproj * a.nb;
+        for (long e = (long)blk * 256 + tid; e < cnt; e += (long)a.nblocks * 256) {
+            const double sw = a.beta[e];
+            en += sw * sw * a.scal2 / a.vnlnrm_p[e / a.nb];
+        }
+        const double t = block_sum<256>(en, sh);
+        if (tid == 0) a.npart[blk] = t;
     }
 }
 
 // hml from M[i][j] = <c1_i|cpsi_j> (row-major per spin), with the reference's
 // mirroring and eorbit reads (cpsd.c:497-515); one thread.
 struct FinalArgs {
-    int ispin, ne0, ne1, nion, nsh, nproj, nb, inner;
-    int pblocks, bblocks, gblocks;
-    const double *ppart, *bpart, *gpart;
+    int ispin, ne0, ne1, nion, nb, inner;
+    int pblocks, bblocks, gblocks, nblocks;
+    const double *ppart, *bpart, *gpart, *npart;
     const double *Mh[2];
     double *hml;
-    const double *beta, *vnlnrm_p;
-    const double *ewald_part;  // real-space Ewald sum per ion (ewald_real_kernel)
-    double scal2, omega, dv, cewald, rcut, dt, dte;
+    const double *ewald_part;  // real-space Ewald sum per ion
+    double scal2, omega, dv, cewald, dt, dte;
     double *E;  // in: E[0] previous energy; out: E[0..9], E[10] deltae, E[11] deltac
 };
-
-// Real-space Ewald sum, cpsd.c:527-545 (A&S 7.1.28 erfc, cpsd.c:11-17): block
-// ii sums the pairs (ii, jj > ii) over the nsh image cells, one (pair, image)
-// term per thread, and writes a fixed-order block sum to part[ii].
-__global__ void __launch_bounds__(256) ewald_real_kernel(int nion, int nsh, const double *__restrict__ r1,
-                                                         const double *__restrict__ rcell,
-                                                         const double *__restrict__ zv,
-                                                         const int *__restrict__ katm, double rcut,
-                                                         double *__restrict__ part)
-{
-    __shared__ double sh[32];
-    const double B1 = 0.0705230784, B2 = 0.0422820123, B3 = 0.0092705272;
-    const double B4 = 0.0001520143, B5 = 0.0002765672, B6 = 0.0000430638;
-    const int ii = blockIdx.x;
-    const long cnt = (long)(nion - 1 - ii) * nsh;
-    double ew = 0.0;
-    for (long e = threadIdx.x; e < cnt; e += 256) {
-        const int jj = ii + 1 + (int)(e / nsh);
-        const int l = (int)(e % nsh);
-        const double dx = r1[3 * ii] - r1[3 * jj];
-        const double dy = r1[1 + 3 * ii] - r1[1 + 3 * jj];
-        const double dz = r1[2 + 3 * ii] - r1[2 + 3 * jj];
-        const double zz = zv[katm[ii]] * zv[katm[jj]];
-        const double x = rcell[l] + dx, y = rcell[l + nsh] + dy, z = rcell[l + 2 * nsh] + dz;
-        const double r = sqrt(x * x + y * y + z * z);
-        const double w = r / rcut;
-        const double aa = (1.0 + w * (B1 + w * (B2 + w * (B3 + w * (B4 + w * (B5 + w * B6))))));
-        const double erfc = 1.0 / (aa * aa * aa * aa);
-        ew += zz * (erfc * erfc * erfc * erfc) / r;
-    }
-    const double t = block_sum<256>(ew, sh);
-    if (threadIdx.x == 0) part[ii] = t;
-}
 
 // One block of kFinalThreads: every sum is a fixed-order block reduction, so
 // the energies are bitwise reproducible run to run.
@@ -1400,7 +1410,7 @@ __global__ void __launch_bounds__(kFinalThreads) final_energy_kernel(FinalArgs a
         for (int k = tid; k < a.pblocks; k += kFinalThreads) v += a.ppart[q * a.pblocks + k];
         t[q] = block_sum<kFinalThreads>(v, sh);
     }
-    // real-space Ewald: per-ion partials of ewald_real_kernel, summed in ion order
+    // real-space Ewald: per-ion partials, summed in ion order
     double eion_real = 0.0;
     if (tid == 0)
         for (int ii = 0; ii < a.nion; ++ii) eion_real += a.ewald_part[ii];
@@ -1436,10 +1446,7 @@ __global__ void __launch_bounds__(kFinalThreads) final_energy_kernel(FinalArgs a
     __syncthreads();
     // nonlocal energy from the last step's projections, cpsd.c:593-634
     double en = 0.0;
-    for (long e = tid; e < (long)a.nproj * a.nb; e += kFinalThreads) {
-        const double sw = a.beta[e];
-        en += sw * sw * a.scal2 / a.vnlnrm_p[e / a.nb];
-    }
+    for (int k = tid; k < a.nblocks; k += kFinalThreads) en += a.npart[k];
     double enl = block_sum<kFinalThreads>(en, sh);
     if (tid != 0) return;
     if (a.ispin == 1) eorbit *= 2;
