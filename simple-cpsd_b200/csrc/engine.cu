@@ -3033,7 +3033,17 @@ int cpsd_gpu_epilogue(cpsd_gpu_ctx *c, double *ortho, double *eig, double *vec)
     ea.eig = c->eigD;
     ea.vec = c->eigVec;
     ea.sweeps = c->eig_sweeps;
-    jacobi_eig_kernel<<<c->ispin, kEigThreads, 0, s>>>(ea);
+    {
+        // (the spins share the launch: sized for the larger one)
+        const int in_smem = eig_in_smem(c->ne0);
+        const size_t smem = sizeof(double) * in_smem * (size_t)c->ne0 * eig_ld(c->ne0);
+        auto run = [&](auto *k, int threads) -> cudaError_t {
+            const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEigSmemMax);
+            if (e == cudaSuccess) k<<<c->ispin, threads, smem, s>>>(ea, in_smem);
+            return e;
+        };
+        CK(c->ne0 <= 32 ? run(jacobi_eig_kernel<256>, 256) : run(jacobi_eig_kernel<1024>, 1024));
+    }
     c->nlaunch += 1;
     // c1 <- c2 V per spin (main.c:481-487): band j of c1 = sum_l V[l][j] band l of c2
     const double *const V[2] = {c->eigVec, c->eigVec + ne02};

@@ -1489,8 +1489,12 @@ __global__ void __launch_bounds__(kFinalThreads) final_energy_kernel(FinalArgs a
 // (S = sum of |a_ij|, i < j) rotate; from the fifth sweep on an a_pq that
 // no longer changes a_pp or a_qq (|a_pp| + 100 |a_pq| == |a_pp|, the same
 // for a_qq) is set to zero.  The sweeps end when S is zero.  One CTA per
-// spin; A and V (column-major, ld n) live in global memory (L2).
-constexpr int kEigThreads = 1024, kEigMaxSweeps = 60;
+// spin.  A round is two dependent phases (the rotations, then every 2 x 2 block
+// of A by a row and a column rotation), so its time is latency: A and V
+// (column-major) live in shared memory where they fit (both up to 110 bands, A
+// alone up to 157), columns an odd stride apart, and up to 32 bands take 256
+// threads (a barrier of 8 warps instead of 32).
+constexpr int kEigMaxSweeps = 60;
 
 struct EigArgs {
     const double *hml;   // per spin ms at hml + ms*ne0*ne0, column-major, ld ne[ms]; upper triangle read
@@ -1501,30 +1505,46 @@ struct EigArgs {
     int *sweeps;         // per spin: sweeps run (kEigMaxSweeps + 1: not converged)
 };
 
-__global__ void __launch_bounds__(kEigThreads) jacobi_eig_kernel(EigArgs a)
+constexpr size_t kEigSmemMax = 200 << 10;
+CPSD_HD int eig_ld(int n) { return n | 1; }
+// matrices held in shared memory: 2 (A and V), 1 (A) or 0
+inline int eig_in_smem(int n)
 {
-    __shared__ double rc[128], rs[128], rapp[128], raqq[128], rt[128], red[32];
-    __shared__ int rp[128], rq[128], perm[256];
+    const size_t one = sizeof(double) * (size_t)n * eig_ld(n);
+    return 2 * one <= kEigSmemMax ? 2 : (one <= kEigSmemMax ? 1 : 0);
+}
+
+template <int kEigThreads>
+__global__ void __launch_bounds__(kEigThreads) jacobi_eig_kernel(EigArgs a, int in_smem)
+{
+    extern __shared__ double eig_sm[];
+    __shared__ double rc[128], rs[128], rd0[128], rd1[128], red[32];
+    __shared__ int rp[128], rq[128], rk[128], perm[256];
     __shared__ double sum_off;
     const int ms = blockIdx.x, n = a.ne[ms], tid = threadIdx.x;
     if (n <= 0) return;
     const long off = (long)ms * a.ne0 * a.ne0;
     const double *H = a.hml + off;
-    double *A = a.A + off, *V = a.V + off;
+    const int la = in_smem >= 1 ? eig_ld(n) : n, lv = in_smem == 2 ? eig_ld(n) : n;  // column strides
+    double *A = in_smem >= 1 ? eig_sm : a.A + off;
+    double *V = in_smem == 2 ? eig_sm + (long)n * la : a.V + off;
     for (long e = tid; e < (long)n * n; e += kEigThreads) {
         const int i = (int)(e % n), j = (int)(e / n);
-        A[e] = (i <= j) ? H[i + (long)j * n] : H[j + (long)i * n];
-        V[e] = (i == j) ? 1.0 : 0.0;
+        A[i + (long)j * la] = (i <= j) ? H[i + (long)j * n] : H[j + (long)i * n];
+        V[i + (long)j * lv] = (i == j) ? 1.0 : 0.0;
     }
     __syncthreads();
     const int np = n + (n & 1), half = np / 2, m1 = np - 1;
+    // a thread's first block (k, l) and V entry (l, i), and its strides
+    const int k0 = tid / half, l0 = tid % half, dk = kEigThreads / half, dl = kEigThreads % half;
+    const int l1 = tid / n, i1 = tid % n, dv = kEigThreads / n, di = kEigThreads % n;
     int sweep = 1;
     for (; sweep <= kEigMaxSweeps; ++sweep) {
         // S = sum_{i<j} |a_ij|
         double v = 0.0;
         for (long e = tid; e < (long)n * n; e += kEigThreads) {
             const int i = (int)(e % n), j = (int)(e / n);
-            if (i < j) v += fabs(A[e]);
+            if (i < j) v += fabs(A[i + (long)j * la]);
         }
         v = block_sum<kEigThreads>(v, red);
         if (tid == 0) sum_off = v;
@@ -1539,24 +1559,24 @@ __global__ void __launch_bounds__(kEigThreads) jacobi_eig_kernel(EigArgs a)
                     p = 0;
                     q = 1 + r;
                 } else {
-                    p = 1 + (r + tid) % m1;
-                    q = 1 + (r - tid + m1) % m1;
+                    p = 1 + (r + tid < m1 ? r + tid : r + tid - m1);
+                    q = 1 + (r >= tid ? r - tid : r - tid + m1);
                 }
                 if (p > q) {
                     const int x = p;
                     p = q;
                     q = x;
                 }
-                double c = 1.0, s = 0.0, t = 0.0;
-                bool rot = false;
+                double c = 1.0, s = 0.0, d0 = 0.0, d1 = 0.0;
+                int kind = 0;  // 0: identity, 1: rotated, 2: a_pq set to zero
                 if (q < n) {
-                    const double app = A[p + (long)p * n], aqq = A[q + (long)q * n], apq = A[p + (long)q * n];
+                    const double app = A[p + (long)p * la], aqq = A[q + (long)q * la], apq = A[p + (long)q * la];
                     const double g = 100.0 * fabs(apq);
                     if (sweep > 4 && fabs(app) + g == fabs(app) && fabs(aqq) + g == fabs(aqq)) {
-                        A[p + (long)q * n] = 0.0;
-                        A[q + (long)p * n] = 0.0;
+                        kind = 2;
                     } else if (fabs(apq) > tresh && apq != 0.0) {
                         const double h = aqq - app;
+                        double t;
                         if (fabs(h) + g == fabs(h)) {
                             t = apq / h;
                         } else {
@@ -1564,64 +1584,76 @@ __global__ void __launch_bounds__(kEigThreads) jacobi_eig_kernel(EigArgs a)
                             t = 1.0 / (fabs(theta) + sqrt(1.0 + theta * theta));
                             if (theta < 0.0) t = -t;
                         }
-                        c = 1.0 / sqrt(1.0 + t * t);
+                        c = rsqrt(1.0 + t * t);
                         s = t * c;
-                        rot = true;
-                        rapp[tid] = app;
-                        raqq[tid] = aqq;
-                        rt[tid] = t * apq;
+                        kind = 1;
+                        d0 = app - t * apq;
+                        d1 = aqq + t * apq;
                     }
                 }
-                rp[tid] = rot ? p : -1;
-                rq[tid] = q;
+                rp[tid] = p;
+                rq[tid] = q;  // n: the idle index of an odd n
+                rk[tid] = kind;
                 rc[tid] = c;
                 rs[tid] = s;
+                rd0[tid] = d0;
+                rd1[tid] = d1;
             }
             __syncthreads();
-            // rows p, q of A: A <- P^T A
-            for (long e = tid; e < (long)half * n; e += kEigThreads) {
-                const int k = (int)(e / n), j = (int)(e % n), p = rp[k];
-                if (p < 0) continue;
-                const int q = rq[k];
-                const double c = rc[k], s = rs[k];
-                const double ap = A[p + (long)j * n], aq = A[q + (long)j * n];
-                A[p + (long)j * n] = c * ap - s * aq;
-                A[q + (long)j * n] = s * ap + c * aq;
+            // A <- P^T A P, one 2 x 2 block (rows of pair k, columns of pair l)
+            // per thread: the rows' rotation, then the columns'.  A rotation's
+            // own block gets a_pp - t a_pq, a_qq + t a_pq and exact zeros.
+            for (int e = tid, k = k0, l = l0; e < half * half; e += kEigThreads) {
+                const int p = rp[k], q = rq[k], u = rp[l], w = rq[l];
+                double *Au = A + (long)u * la, *Aw = A + (long)w * la;
+                if (k == l) {
+                    if (rk[k] == 1) {
+                        Au[p] = rd0[k];
+                        Aw[q] = rd1[k];
+                    }
+                    if (rk[k] != 0) {
+                        Aw[p] = 0.0;
+                        Au[q] = 0.0;
+                    }
+                } else if (rk[k] == 1 || rk[l] == 1) {
+                    const double c = rc[k], sn = rs[k], c2 = rc[l], s2 = rs[l];
+                    const bool hq = q < n, hw = w < n;
+                    const double pu = Au[p], qu = hq ? Au[q] : 0.0, pw = hw ? Aw[p] : 0.0, qw = (hq && hw) ? Aw[q] : 0.0;
+                    const double x0 = c * pu - sn * qu, x1 = sn * pu + c * qu;  // column u
+                    const double y0 = c * pw - sn * qw, y1 = sn * pw + c * qw;  // column w
+                    Au[p] = c2 * x0 - s2 * y0;
+                    if (hq) Au[q] = c2 * x1 - s2 * y1;
+                    if (hw) Aw[p] = s2 * x0 + c2 * y0;
+                    if (hq && hw) Aw[q] = s2 * x1 + c2 * y1;
+                }
+                k += dk;
+                l += dl;
+                if (l >= half) {
+                    l -= half;
+                    ++k;
+                }
             }
-            __syncthreads();
-            // columns p, q of A and V: A <- A P, V <- V P
-            for (long e = tid; e < (long)half * n; e += kEigThreads) {
-                const int k = (int)(e / n), i = (int)(e % n), p = rp[k];
-                if (p < 0) continue;
-                const int q = rq[k];
-                const double c = rc[k], s = rs[k];
-                double *cp = A + (long)p * n, *cq = A + (long)q * n;
-                double x = cp[i], y = cq[i];
-                cp[i] = c * x - s * y;
-                cq[i] = s * x + c * y;
-                cp = V + (long)p * n;
-                cq = V + (long)q * n;
-                x = cp[i];
-                y = cq[i];
-                cp[i] = c * x - s * y;
-                cq[i] = s * x + c * y;
-            }
-            __syncthreads();
-            // the rotated 2 x 2 blocks (touched by their own rotation only):
-            // a_pp - t a_pq, a_qq + t a_pq and exact zeros off the diagonal
-            if (tid < half && rp[tid] >= 0) {
-                const int p = rp[tid], q = rq[tid];
-                A[p + (long)p * n] = rapp[tid] - rt[tid];
-                A[q + (long)q * n] = raqq[tid] + rt[tid];
-                A[p + (long)q * n] = 0.0;
-                A[q + (long)p * n] = 0.0;
+            // V <- V P
+            for (int e = tid, l = l1, i = i1; e < half * n; e += kEigThreads) {
+                if (rk[l] == 1) {
+                    double *cp = V + (long)rp[l] * lv, *cq = V + (long)rq[l] * lv;
+                    const double c = rc[l], sn = rs[l], x = cp[i], y = cq[i];
+                    cp[i] = c * x - sn * y;
+                    cq[i] = sn * x + c * y;
+                }
+                l += dv;
+                i += di;
+                if (i >= n) {
+                    i -= n;
+                    ++l;
+                }
             }
             __syncthreads();
         }
         // restore exact symmetry from the upper triangle
         for (long e = tid; e < (long)n * n; e += kEigThreads) {
             const int i = (int)(e % n), j = (int)(e / n);
-            if (i > j) A[e] = A[j + (long)i * n];
+            if (i > j) A[i + (long)j * la] = A[j + (long)i * la];
         }
         __syncthreads();
     }
@@ -1630,9 +1662,9 @@ __global__ void __launch_bounds__(kEigThreads) jacobi_eig_kernel(EigArgs a)
         for (int i = 0; i < n; ++i) perm[i] = i;
         for (int i = 0; i < n - 1; ++i) {
             int k = i;
-            double p = A[perm[i] + (long)perm[i] * n];
+            double p = A[perm[i] + (long)perm[i] * la];
             for (int j = i + 1; j < n; ++j) {
-                const double d = A[perm[j] + (long)perm[j] * n];
+                const double d = A[perm[j] + (long)perm[j] * la];
                 if (d >= p) {
                     k = j;
                     p = d;
@@ -1647,9 +1679,9 @@ __global__ void __launch_bounds__(kEigThreads) jacobi_eig_kernel(EigArgs a)
         a.sweeps[ms] = sweep;
     }
     __syncthreads();
-    for (int i = tid; i < n; i += kEigThreads) a.eig[(long)ms * a.ne0 + i] = A[perm[i] + (long)perm[i] * n];
+    for (int i = tid; i < n; i += kEigThreads) a.eig[(long)ms * a.ne0 + i] = A[perm[i] + (long)perm[i] * la];
     for (long e = tid; e < (long)n * n; e += kEigThreads) {
         const int i = (int)(e % n), j = (int)(e / n);
-        a.vec[off + i + (long)j * n] = V[i + (long)perm[j] * n];
+        a.vec[off + i + (long)j * n] = V[i + (long)perm[j] * lv];
     }
 }
