@@ -92,7 +92,7 @@ struct HostGeom {
     // with q): host loops over the reference's grids walk them in memory
     // order instead of one column (stride nh*n) at a time
     std::vector<int> pt_ord;
-    int span = 0;           // lines that can be nonzero on either side of k = 0: kx < span, |ky| < span
+    int span = 0;           // lines that can be nonzero on either side of k = 0: kx, |ky|, |kz| < span
     std::vector<int> yrun;  // 3 per line kx < KX (see Geom::yrun), empty if some line is not two runs
     std::vector<double> w;
 };
@@ -132,7 +132,8 @@ HostGeom build_geom(int n, const int *masker1, bool full)
     h.ncol = (int)h.col_i.size();
     h.npw = (int)h.pt_k.size();
     h.span = h.KX;
-    for (int j : h.col_j) h.span = std::max(h.span, j <= n / 2 ? j + 1 : n - j);
+    for (const auto *v : {&h.col_j, &h.pt_k})
+        for (int j : *v) h.span = std::max(h.span, j <= n / 2 ? j + 1 : n - j);
     h.pt_ord.reserve(h.npw);
     for (long idx = 0; idx < nfft3d; ++idx)
         if (h.inv_idx[idx] >= 0) h.pt_ord.push_back(h.inv_idx[idx]);
@@ -320,6 +321,15 @@ struct FftOpsT final : FftOps {
         return f(pair_kernel<T, NF, MODE, Line<NF>::Q / 2>);
     }
 
+    // f(KZ) for the z passes
+    template <typename F>
+    cudaError_t with_z(F &&f)
+    {
+        if constexpr (kKZ > 0)
+            if (pruned) return f(std::integral_constant<int, kKZ>{});
+        return f(std::integral_constant<int, Line<NF>::Q / 2>{});
+    }
+
     template <int MODE>
     int init_pair(int ncol, int optin)
     {
@@ -388,9 +398,17 @@ struct FftOpsT final : FftOps {
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
         static_assert(zpot_smem_bytes<T, NF>() <= 48 << 10, "no opt-in shared memory");
-        CK(cudaFuncSetAttribute(inv_z_kernel<T, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem));
-        CK(cudaFuncSetAttribute(fwd_z_kernel<T, NF, ZEPI_STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem));
-        CK(cudaFuncSetAttribute(fwd_z_kernel<T, NF, ZEPI_SD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem));
+        cudaError_t e = with_z([&](auto kz) {
+            constexpr int KZ = decltype(kz)::value;
+            const void *k[3] = {(const void *)inv_z_kernel<T, NF, KZ>, (const void *)fwd_z_kernel<T, NF, ZEPI_STORE, KZ>,
+                                (const void *)fwd_z_kernel<T, NF, ZEPI_SD, KZ>};
+            for (const void *x : k) {
+                const cudaError_t r = cudaFuncSetAttribute(x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem);
+                if (r != cudaSuccess) return r;
+            }
+            return cudaSuccess;
+        });
+        CK(e);
         for (int m = 0; m < 4; ++m) {
             psmem[m] = plane_smem_bytes<T, NF>(m, KX, ncol, 2);
             psmem1[m] = plane_smem_bytes<T, NF>(m, KX, ncol, 1);
@@ -462,7 +480,10 @@ struct FftOpsT final : FftOps {
     {
         constexpr int CPB = kThreads / Line<NF>::P;
         dim3 grid((unsigned)cdiv(g.ncol, CPB), (unsigned)nb);
-        launch(inv_z_kernel<T, NF>, grid, kThreads, zsmem, s, chain, g, psi, ldp, (cx<T> *)Tb, tw);
+        (void)with_z([&](auto kz) {
+            launch(inv_z_kernel<T, NF, decltype(kz)::value>, grid, kThreads, zsmem, s, chain, g, psi, ldp, (cx<T> *)Tb, tw);
+            return cudaSuccess;
+        });
     }
     void fwd_z_store(const Geom &g, const void *Tb, cx<double> *out, long ldo, double scale, int nb,
                      cudaStream_t s) override
@@ -473,13 +494,19 @@ struct FftOpsT final : FftOps {
         e.ldo = ldo;
         e.scale = scale;
         dim3 grid((unsigned)cdiv(g.ncol, CPB), (unsigned)nb);
-        fwd_z_kernel<T, NF, ZEPI_STORE><<<grid, kThreads, zsmem, s>>>(g, (const cx<T> *)Tb, e, tw);
+        (void)with_z([&](auto kz) {
+            fwd_z_kernel<T, NF, ZEPI_STORE, decltype(kz)::value><<<grid, kThreads, zsmem, s>>>(g, (const cx<T> *)Tb, e, tw);
+            return cudaSuccess;
+        });
     }
     void fwd_z_sd(const Geom &g, const void *Tb, const ZEpilogue &e, int nb, cudaStream_t s) override
     {
         constexpr int CPB = kThreads / Line<NF>::P;
         dim3 grid((unsigned)cdiv(g.ncol, CPB), (unsigned)nb);
-        fwd_z_kernel<T, NF, ZEPI_SD><<<grid, kThreads, zsmem, s>>>(g, (const cx<T> *)Tb, e, tw);
+        (void)with_z([&](auto kz) {
+            fwd_z_kernel<T, NF, ZEPI_SD, decltype(kz)::value><<<grid, kThreads, zsmem, s>>>(g, (const cx<T> *)Tb, e, tw);
+            return cudaSuccess;
+        });
     }
     void z_potential(const Geom &g, void *Tb, const ZPotArgs &a, cudaStream_t s, bool chain) override
     {

@@ -23,95 +23,7 @@
 #pragma once
 
 #include "fft.cuh"
-
-// In-register DFT of size N whose inputs outside MASK are zero (not read).
-template <int N, int SIGN, typename T, unsigned MASK>
-struct DFTM;
-
-template <bool A, bool B, typename T>
-CPSD_D cx<T> addz(cx<T> a, cx<T> b)
-{
-    if constexpr (A && B) return a + b;
-    else if constexpr (A) return a;
-    else if constexpr (B) return b;
-    else return cx<T>{0, 0};
-}
-template <bool A, bool B, typename T>
-CPSD_D cx<T> subz(cx<T> a, cx<T> b)
-{
-    if constexpr (A && B) return a - b;
-    else if constexpr (A) return a;
-    else if constexpr (B) return cx<T>{-b.x, -b.y};
-    else return cx<T>{0, 0};
-}
-
-template <int SIGN, typename T, unsigned MASK>
-struct DFTM<2, SIGN, T, MASK> {
-    CPSD_D static void run(cx<T> *v)
-    {
-        constexpr bool A = MASK & 1, B = MASK & 2;
-        cx<T> a = v[0], b = v[1];
-        v[0] = addz<A, B>(a, b);
-        v[1] = subz<A, B>(a, b);
-    }
-};
-template <int SIGN, typename T, unsigned MASK>
-struct DFTM<4, SIGN, T, MASK> {
-    CPSD_D static void run(cx<T> *v)
-    {
-        constexpr bool A = MASK & 1, B = MASK & 2, C = MASK & 4, D = MASK & 8;
-        cx<T> a = v[0], b = v[1], c = v[2], d = v[3];
-        const cx<T> s0 = addz<A, C>(a, c), s1 = subz<A, C>(a, c), s2 = addz<B, D>(b, d);
-        const cx<T> s3 = mul_is<SIGN>(subz<B, D>(b, d));
-        v[0] = addz<A || C, B || D>(s0, s2);
-        v[1] = addz<A || C, B || D>(s1, s3);
-        v[2] = subz<A || C, B || D>(s0, s2);
-        v[3] = subz<A || C, B || D>(s1, s3);
-    }
-};
-// inputs r, r + R, r + 2 R, ... of the size-N mask
-template <int N, int R>
-constexpr unsigned dft_sub_mask(unsigned mask, int r)
-{
-    unsigned s = 0;
-    for (int m = 0; m < N / R; ++m) s |= ((mask >> (r + R * m)) & 1u) << m;
-    return s;
-}
-template <int N, int SIGN, typename T, unsigned MASK>
-struct DFTM {
-    CPSD_D static void run(cx<T> *v)
-    {
-        if constexpr (MASK == (N >= 32 ? ~0u : (1u << N) - 1u)) {
-            DFT<N, SIGN, T>::run(v);
-        } else {
-            constexpr int R = 4, M = N / 4;  // 8 = 4 x 2, 16 = 4 x 4
-            static_assert(N == 8 || N == 16, "masked DFT size");
-            cx<T> sub[R][M];
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-#pragma unroll
-                for (int m = 0; m < M; ++m) sub[r][m] = v[r + R * m];
-            SFor<0, R>::run([&](auto rc) {
-                constexpr int r = decltype(rc)::value;
-                constexpr unsigned sm = dft_sub_mask<N, R>(MASK, r);
-                if constexpr (sm != 0) DFTM<M, SIGN, T, sm>::run(sub[r]);
-            });
-            constexpr unsigned top = (dft_sub_mask<N, R>(MASK, 0) ? 1u : 0u) | (dft_sub_mask<N, R>(MASK, 1) ? 2u : 0u) |
-                                     (dft_sub_mask<N, R>(MASK, 2) ? 4u : 0u) | (dft_sub_mask<N, R>(MASK, 3) ? 8u : 0u);
-            SFor<0, M>::run([&](auto kc) {
-                constexpr int k = decltype(kc)::value;
-                cx<T> t[R];
-                SFor<0, R>::run([&](auto rc) {
-                    constexpr int r = decltype(rc)::value;
-                    if constexpr ((top >> r) & 1u) t[r] = twmul<N, SIGN, r * k>(sub[r][k]);
-                });
-                DFTM<R, SIGN, T, top>::run(t);
-#pragma unroll
-                for (int q = 0; q < R; ++q) v[k + M * q] = t[q];
-            });
-        }
-    }
-};
+#include "lines.cuh"
 
 // Twiddles of the pair passes, one allocation: the inverse lines' table in
 // line_fft's order (q P + t), and the forward (transposed) lines' table,
@@ -176,68 +88,6 @@ size_t pair_smem_bytes(int KX, int ncol, bool stage)
     return (b + 15) / 16 * 16;
 }
 
-// One exchange of a line: lane t stores its Q values at the slots sidx(i) and
-// loads Q values from lidx(i); real and imaginary parts in turn when SPLIT.
-template <int Q, bool SPLIT, typename T, typename SI, typename LI>
-CPSD_D void pair_exchange(cx<T> *v, void *buf, SI sidx, LI lidx)
-{
-    if constexpr (SPLIT) {
-        T *b = static_cast<T *>(buf);
-#pragma unroll
-        for (int i = 0; i < Q; ++i) b[sidx(i)] = v[i].x;
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < Q; ++i) v[i].x = b[lidx(i)];
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < Q; ++i) b[sidx(i)] = v[i].y;
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < Q; ++i) v[i].y = b[lidx(i)];
-        __syncwarp();
-    } else {
-        cx<T> *b = static_cast<cx<T> *>(buf);
-#pragma unroll
-        for (int i = 0; i < Q; ++i) b[sidx(i)] = v[i];
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < Q; ++i) v[i] = b[lidx(i)];
-        __syncwarp();
-    }
-}
-
-// The passes at n = 128 are bound by shared memory (70 % of its wavefronts
-// busy in V psi, FP64 pipe 43 %), so half of a lane's twiddles are formed by a
-// product instead of read: V psi 0.856 -> 0.813 ms, density 0.537 -> 0.524 ms
-// (FP64), 0.340 -> 0.323 ms (FP32 density); the error against 64 bits stays.
-
-// line_fft (common.cuh) with masked inputs: x[t + P m] in v[m] -> X[(t U + u)
-// + Q s] in v[u P + s], sign +1.
-template <int N, typename T, unsigned MASK, bool SPLIT>
-CPSD_D void pair_inverse(cx<T> *v, int t, void *xb, const cx<T> *__restrict__ tw)
-{
-    using L = Line<N>;
-    constexpr int P = L::P, Q = L::Q, U = L::U;
-    DFTM<Q, +1, T, MASK>::run(v);
-    if constexpr (Q == 16) {  // W^(q + 8) t from two table entries (see above)
-        const cx<T> w8 = tw[8 * P + t];
-        v[8] = cmul(v[8], w8);
-#pragma unroll
-        for (int q = 1; q < 8; ++q) {
-            const cx<T> w = tw[q * P + t];
-            v[q] = cmul(v[q], w);
-            v[q + 8] = cmul(v[q + 8], cmul(w, w8));
-        }
-    } else {
-#pragma unroll
-        for (int q = 1; q < Q; ++q) v[q] = cmul(v[q], tw[q * P + t]);
-    }
-    pair_exchange<Q, SPLIT>(v, xb, [t](int q) { return L::xb_index(q, t); },
-                            [t](int i) { return L::xb_index(t * U + i / P, i % P); });
-#pragma unroll
-    for (int u = 0; u < U; ++u) DFT<P, +1, T>::run(v + u * P);
-}
-
 // line_fft_dif with the pair passes' table: x[(t U + u) + Q s] in v[u P + s]
 // -> X[t + P m] in v[m], sign -1.
 template <int N, typename T, bool SPLIT>
@@ -262,7 +112,7 @@ CPSD_D void pair_forward(cx<T> *v, int t, void *xb, const cx<T> *__restrict__ tw
             for (int tp = 1; tp < P; ++tp) v[u * P + tp] = cmul(v[u * P + tp], tw[(tp * U + u) * P + t]);
         }
     }
-    pair_exchange<Q, SPLIT>(v, xb, [t](int i) { return L::xb_index(t * U + i / P, i % P); },
+    line_exchange<Q, SPLIT>(v, xb, [t](int i) { return L::xb_index(t * U + i / P, i % P); },
                             [t](int q) { return L::xb_index(q, t); });
     DFT<Q, -1, T>::run(v);
 }
@@ -286,7 +136,7 @@ pair_kernel(Geom g, cx<T> *__restrict__ Tb, PairArgs a, const cx<T> *__restrict_
     constexpr int P = L::P, Q = L::Q, U = L::U, H = NF / 2;
     constexpr int NT = C::NT, NG = C::NG, YS = S::YS;
     constexpr bool ALL = 2 * KZ >= Q;
-    constexpr unsigned MASK = ALL ? (1u << Q) - 1u : ((1u << KZ) - 1u) | (((1u << KZ) - 1u) << (Q - KZ));
+    constexpr unsigned MASK = line_mask<Q, KZ>();
     constexpr int NIT = (NF + NG - 1) / NG;  // x rows per group
     extern __shared__ unsigned char smem_raw[];
     const int KX = g.KX, ncol = g.ncol;
@@ -359,7 +209,7 @@ pair_kernel(Geom g, cx<T> *__restrict__ Tb, PairArgs a, const cx<T> *__restrict_
                     v[m] = (c < 0) ? cx<T>{0, 0} : (a.stage ? sst[c] : src[c]);
                 }
             });
-            pair_inverse<NF, T, MASK, C::SPLIT>(v, t, xb, twi);
+            line_masked<NF, +1, T, MASK, C::SPLIT>(v, t, xb, twi);
             if (act) {
                 cx<T> *Yl = Y + li * YS;
 #pragma unroll
@@ -399,7 +249,7 @@ pair_kernel(Geom g, cx<T> *__restrict__ Tb, PairArgs a, const cx<T> *__restrict_
                         v[m] = cx<T>{xa.x + xc.y, xc.x - xa.y};
                 }
             });
-            pair_inverse<NF, T, MASK, C::SPLIT>(v, t, xb, twi);
+            line_masked<NF, +1, T, MASK, C::SPLIT>(v, t, xb, twi);
             // v[u P + s] = (psi_A(x), psi_B(x)), x = (t U + u) + Q s
             if constexpr (MODE == PM_DENSITY) {
 #pragma unroll
