@@ -1337,6 +1337,16 @@ cudaError_t copy_positions(cpsd_gpu_ctx *c, cudaStream_t s)
     return cudaMemcpyAsync(c->r1, c->r2, sizeof(double) * 3 * c->nion, cudaMemcpyDeviceToDevice, s);
 }
 
+// the tiled solver's build for the larger spin's bands
+void (*lagrange_tile(int ne0))(LagArgs)
+{
+    switch (lag_tile_mt(ne0)) {
+    case 1: case 2: return lagrange_tile_kernel<2>;
+    case 3: return lagrange_tile_kernel<3>;
+    default: return lagrange_tile_kernel<4>;
+    }
+}
+
 // One SD step in three phases.  A context that steps every band runs them
 // back to back (one_step); a band-parallel context (c->bp) steps only its
 // bands [bp_lo, bp_hi) in phases 0 and 1, and its caller exchanges between
@@ -1598,7 +1608,7 @@ int step_phase(cpsd_gpu_ctx *c, int phase)
         cfg.stream = s;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        CK(cudaLaunchKernelEx(&cfg, lagrange_tile_kernel, la));
+        CK(cudaLaunchKernelEx(&cfg, lagrange_tile(c->ne0), la));
     } else {
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute attr[1];
@@ -2795,8 +2805,8 @@ int cpsd_gpu_create(const cpsd_gpu_params *p, const int *masker1, cpsd_gpu_ctx *
         const char *lag_env = getenv("CPSD_B200_LAGRANGE");
         const size_t tsm = lagrange_tile_smem(c->ne0);
         if (c->ne0 <= kLagTileMax && tsm <= limit) {
-            CK(cudaFuncSetAttribute(lagrange_tile_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            CK(allow_max_smem(lagrange_tile_kernel, optin));
+            CK(cudaFuncSetAttribute(lagrange_tile(c->ne0), cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            CK(allow_max_smem(lagrange_tile(c->ne0), optin));
             cudaLaunchConfig_t cfg{};
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -2809,7 +2819,7 @@ int cpsd_gpu_create(const cpsd_gpu_params *p, const int *masker1, cpsd_gpu_ctx *
             cfg.attrs = attr;
             cfg.numAttrs = 1;
             int nclusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&nclusters, lagrange_tile_kernel, &cfg) == cudaSuccess &&
+            if (cudaOccupancyMaxActiveClusters(&nclusters, lagrange_tile(c->ne0), &cfg) == cudaSuccess &&
                 nclusters >= 1)
                 c->lag_tile_ok = true;
             (void)cudaGetLastError();

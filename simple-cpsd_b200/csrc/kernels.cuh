@@ -1015,229 +1015,244 @@ __global__ void __launch_bounds__(kLagThreads) lagrange_kernel(LagArgs a)
 // up to this many bands per spin: small.cuh
 constexpr int kLagSmallMax = 32;
 
-// ------------------------------------------------- Lagrange, 2-D tiles
-// lagrange_tile_kernel: the same fixed point as lagrange_kernel (cpsd.c:
-// 439-478, including the idamax read and the 30-iteration limit) for up to
-// 128 bands per spin, on a cluster of 4 x 4 CTAs.  CTA (p, q) owns the tile
-// rows I_p x columns J_q (T = ceil(m / 4) of each) of sa0, sa1 and st1, and
-// keeps its constant panels s21[I_p, :], s11[I_p, :], s12[:, J_q] and
-// s22[I_p, J_q] in shared memory for all iterations.  Per iteration:
-//   phase 1: gather sa0[I_p, :] and sa0[:, J_q] from the tiles of its row and
-//            column (distributed shared memory), t = s22 + s21 sa0 + sa0 s12,
-//            st1 = s11 sa0 on its tile;               cluster barrier;
-//   phase 2: gather st1[:, J_q], sa1 = t + sa0 st1, st1 = sa1 - sa0, the
-//            tile's argmax of |st1|;                  cluster barrier;
-// then every CTA reduces the 16 candidates in rank order and reads the
-// element after the maximum, as the reference does.  sa1 goes into the
-// other half of a double-buffered tile, so the two barriers are all an
-// iteration needs.
-constexpr int kLagTileGrid = 4;  // 4 x 4 CTAs
-constexpr int kLagTileMax = 128;
-
-CPSD_HD size_t lagrange_tile_smem(int m)
+// largest |d| over a warp with the smallest index among equals, as idamax
+// (NaN never wins; 0x7fffffff where every entry was NaN); all lanes get the result
+CPSD_D void combine_argmax(unsigned h, unsigned l, unsigned idx, unsigned &hi, unsigned &lo, int &at)
 {
-    const size_t T = (size_t)(m + kLagTileGrid - 1) / kLagTileGrid;
-    // S21r, S11r, S12c, Xr, Xc, STc: m*T each; S22t, STt: T*T; Xt: 2*T*T; slots
-    return sizeof(double) * (6 * (size_t)m * T + 4 * T * T + 2 * kLagTileGrid * kLagTileGrid);
+    hi = __reduce_max_sync(0xffffffffu, h);
+    lo = __reduce_max_sync(0xffffffffu, h == hi ? l : 0u);
+    at = (int)__reduce_min_sync(0xffffffffu, (h == hi && l == lo) ? idx : 0x7fffffffu);
+}
+CPSD_D void warp_argmax(double ad, int idx, unsigned &hi, unsigned &lo, int &at)
+{
+    const bool ok = ad >= 0.0;  // false for NaN and for "no entry" (-1)
+    const unsigned long long k = ok ? (unsigned long long)__double_as_longlong(ad) : 0ull;
+    combine_argmax((unsigned)(k >> 32), (unsigned)k, ok ? (unsigned)idx : 0x7fffffffu, hi, lo, at);
 }
 
+// ------------------------------------------------- Lagrange, 2-D tiles
+// lagrange_tile_kernel: the same fixed point as lagrange_kernel (cpsd.c:
+// 439-478, including the idamax read and the 30-iteration limit) for 33 to
+// 128 bands per spin, on a cluster of 4 x 4 CTAs.  CTA (p, q) owns the tile
+// rows I_p x columns J_q (T = 8 MT of each, zero padded) of sa0 and sa1, keeps
+// its constant panels s21[I_p, :], s11[I_p, :] and s12[:, J_q]' in shared
+// memory and forms its products on the FP64 tensor cores (8 x 8 tiles, a warp
+// has up to two of one row).  The CTAs push what the others need into their
+// shared memory: st1 = s11 sa0 to the CTAs of its column after the first
+// phase, the new sa0 to those of its row and its column after the second, so
+// every operand is read from local memory:
+//   phase 1: t = s22 + s21 sa0 + sa0 s12, st1 = s11 sa0;   cluster barrier;
+//   phase 2: sa1 = t + sa0 st1 (sa0's rows still in registers), st1 = sa1 -
+//            sa0, the tile's argmax of |st1|;              cluster barrier;
+// then every CTA reduces the 16 candidates and reads the element after the
+// maximum, as the reference does.  All panels are stored with k along the row
+// (the column panels transposed), 8 mod 16 reals apart: fragment loads of two
+// k-steps are 16 bytes and free of bank conflicts.
+//
+// Bound at 128 bands: the FP64 pipe of 16 SMs, 8,192 cycles (4.2 us) an
+// iteration; a solve takes 131 us with CUDA-core products and panels gathered
+// from the peers, 70 us here (40 bands at 32^3: ten steps 1.26 -> 1.10 ms).
+constexpr int kLagTileGrid = 4;  // 4 x 4 CTAs
+constexpr int kLagTileMax = 128;
+constexpr int lag_tile_ld(int mt) { return 32 * mt + 8; }
+
+inline int lag_tile_mt(int m) { return (m + 31) / 32; }  // tiles of 8 along a CTA's edge
+inline size_t lagrange_tile_smem(int m)
+{
+    const int mt = lag_tile_mt(m);
+    // S21r, S11r, S12c, Xr, Xc, STc
+    return sizeof(double) * 6 * (size_t)(8 * mt) * lag_tile_ld(mt);
+}
+
+template <int MT>
 __global__ void __launch_bounds__(kLagThreads) lagrange_tile_kernel(LagArgs a)
 {
+    constexpr int T = 8 * MT, MP = 4 * T, LD = lag_tile_ld(MT), KB = MP / 8, CPW = (MT + 1) / 2, G = kLagTileGrid;
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
-    const int p = rank / kLagTileGrid, q = rank % kLagTileGrid;
-    const int tid = threadIdx.x;
-    extern __shared__ double tsm[];
+    const int p = rank / G, q = rank % G;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, fr = lane >> 2, fq = lane & 3;
+    extern __shared__ __align__(16) double tsm[];
+    __shared__ unsigned slot[G * G][4];  // every CTA's candidate
+    __shared__ unsigned wslot[kLagThreads / 32][4];
     const long ne02 = (long)a.ne0 * a.ne0;
-    const int T = (a.ne0 + kLagTileGrid - 1) / kLagTileGrid;  // tile edge (sized for the larger spin)
-    double *S21r = tsm, *S11r = S21r + (long)a.ne0 * T, *S12c = S11r + (long)a.ne0 * T;
-    double *Xr = S12c + (long)a.ne0 * T, *Xc = Xr + (long)a.ne0 * T, *STc = Xc + (long)a.ne0 * T;
-    double *S22t = STc + (long)a.ne0 * T, *STt = S22t + T * T, *Xt = STt + T * T;  // Xt: two halves
-    double *slot = Xt + 2 * T * T;                                                 // [rank][2]
+    double *S21r = tsm, *S11r = S21r + T * LD, *S12c = S11r + T * LD, *Xr = S12c + T * LD, *Xc = Xr + T * LD,
+           *STc = Xc + T * LD;
+    // this warp's tiles: row tile wi, column tiles wj .. wj + CPW - 1
+    const int wi = warp >> 1, wj = (warp & 1) * CPW;
+    const bool wact = wi < MT;
+    const int i = 8 * wi + fr;  // this lane's row of the CTA's tile
+    double *xr_to[G], *xc_to[G], *st_to[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        xr_to[g] = cl.map_shared_rank(Xr, p * G + g);
+        xc_to[g] = cl.map_shared_rank(Xc, g * G + q);
+        st_to[g] = cl.map_shared_rank(STc, g * G + q);
+    }
     for (int ms = 0; ms < a.ispin; ++ms) {
         const int m = ms ? a.ne1 : a.ne0;
         const long kk = (long)m * m;
         if (m == 0) continue;
-        const int t = (m + kLagTileGrid - 1) / kLagTileGrid;  // this spin's tile edge
-        const int i0 = p * t, j0 = q * t;
-        const int nr = max(0, min(m, i0 + t) - i0), nc = max(0, min(m, j0 + t) - j0);
+        const int i0 = p * T, j0 = q * T;
         const double *M22 = a.M22[ms], *M21 = a.M21[ms], *M11 = a.M11[ms];
         const double dte = a.dte;
         // s matrices, cpsd.c:420-437 (upper triangles mirrored as the reference does)
-        for (long e = (long)rank * kLagThreads + tid; e < kk; e += (long)kLagTileGrid * kLagTileGrid * kLagThreads) {
-            const int i = (int)(e % m), j = (int)(e / m);
-            double v22, v21, v12, v11;
-            if (i == j) {
-                v22 = (1.0 - M22[(long)i * m + i]) * 0.5 / dte;
-                v21 = (1.0 - M21[(long)i * m + i]) * 0.5;
-                v12 = v21;
-                v11 = -M11[(long)i * m + i] * 0.5 * dte;
-            } else {
-                const int lo = i < j ? i : j, hi = i < j ? j : i;
-                v22 = -M22[(long)lo * m + hi] * 0.5 / dte;
-                v21 = -M21[(long)lo * m + hi] * 0.5;   // <c2_lo|c1_hi>
-                v12 = -M21[(long)hi * m + lo] * 0.5;   // <c1_lo|c2_hi>
+        auto s22 = [&](int r, int c) {
+            if (r >= m || c >= m) return 0.0;
+            return r == c ? (1.0 - M22[(long)r * m + r]) * 0.5 / dte : -M22[(long)min(r, c) * m + max(r, c)] * 0.5 / dte;
+        };
+        for (int e = tid; e < T * MP; e += kLagThreads) {
+            const int r = e / MP, l = e % MP, ri = i0 + r, cj = j0 + r;
+            double v21 = 0.0, v11 = 0.0, v12 = 0.0;
+            if (l < m && ri < m) {
+                const int lo = min(ri, l), hi = max(ri, l);
+                v21 = ri == l ? (1.0 - M21[(long)ri * m + ri]) * 0.5 : -M21[(long)lo * m + hi] * 0.5;  // <c2_lo|c1_hi>
                 v11 = -M11[(long)lo * m + hi] * 0.5 * dte;
             }
-            a.s22[e] = v22;
-            a.s21[e] = v21;
-            a.s12[e] = v12;
-            a.s11[e] = v11;
+            if (l < m && cj < m) {
+                const int lo = min(cj, l), hi = max(cj, l);
+                v12 = cj == l ? (1.0 - M21[(long)cj * m + cj]) * 0.5 : -M21[(long)hi * m + lo] * 0.5;  // <c1_lo|c2_hi>
+            }
+            S21r[r * LD + l] = v21;
+            S11r[r * LD + l] = v11;
+            S12c[r * LD + l] = v12;
+            Xr[r * LD + l] = s22(ri, l);  // sa0 = s22, cpsd.c:441
+            Xc[r * LD + l] = s22(l, cj);
         }
-        cl.sync();
-        // constant panels; sa0 = s22 (cpsd.c:441) into the first half of Xt
-        for (int e = tid; e < m * t; e += kLagThreads) {
-            const int l = e / t, ii = e % t;
-            S21r[l * t + ii] = ii < nr ? a.s21[(i0 + ii) + (long)l * m] : 0.0;
-            S11r[l * t + ii] = ii < nr ? a.s11[(i0 + ii) + (long)l * m] : 0.0;
-            const int jj = e % t;
-            S12c[l * t + jj] = jj < nc ? a.s12[l + (long)(j0 + jj) * m] : 0.0;
-        }
-        for (int e = tid; e < t * t; e += kLagThreads) {
-            const int jj = e / t, ii = e % t;
-            const double v = (ii < nr && jj < nc) ? a.s22[(i0 + ii) + (long)(j0 + jj) * m] : 0.0;
-            S22t[jj * t + ii] = v;
-            Xt[jj * t + ii] = v;
-        }
-        // thread -> one row ii of the tile and 4 of its columns
-        const int ii = tid % 32, jq = (tid / 32) * 4;
-        const bool rowok = ii < nr;
-        int half = 0;  // which half of Xt holds sa0
+        double c22[CPW][2], x[CPW][2];
+#pragma unroll
+        for (int u = 0; u < CPW; ++u)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const bool ok = wact && wj + u < MT;
+                x[u][e] = c22[u][e] = ok ? s22(i0 + i, j0 + 8 * (wj + u) + 2 * fq + e) : 0.0;
+            }
         bool done = false;
         int iter = 0;
-        cl.sync();  // every tile's sa0 is in place (later: ordered by the candidates' barrier)
+        cl.sync();  // every CTA's panels are in place (and, for spin 1, spin 0's reads done)
         while (!done && iter < 30) {
             ++iter;
-            // gather sa0[I_p, :] (Xr, [l][ii]) and sa0[:, J_q] (Xc, [l][jj])
-            for (int g = 0; g < kLagTileGrid; ++g) {
-                const double *rowt = cl.map_shared_rank(Xt + half * t * t, p * kLagTileGrid + g);
-                const double *colt = cl.map_shared_rank(Xt + half * t * t, g * kLagTileGrid + q);
-                for (int e = tid; e < t * t; e += kLagThreads) {
-                    const int c = e / t, r = e % t;  // tile element (r, c), stored [c][r]
-                    const int lr = g * t + c, lc = g * t + r;
-                    if (lr < m) Xr[lr * t + r] = rowt[e];
-                    if (lc < m) Xc[lc * t + c] = colt[e];
-                }
-            }
-            __syncthreads();
-            // t = s22 + s21 sa0 + sa0 s12 ; st1 = s11 sa0   (cpsd.c:444-462)
-            double t1[4], t2[4], st[4];
+            double2 xa[KB];
+            double part[CPW][2];
+            if (wact) {
+                const double *xrow = Xr + i * LD + 2 * fq, *s21 = S21r + i * LD + 2 * fq, *s11 = S11r + i * LD + 2 * fq;
+                double t1[CPW][2] = {}, t2[CPW][2] = {}, st[CPW][2] = {};
 #pragma unroll
-            for (int k = 0; k < 4; ++k) t1[k] = t2[k] = st[k] = 0.0;
-            if (rowok)
-                for (int l = 0; l < m; ++l) {
-                    const double a21 = S21r[l * t + ii], a11 = S11r[l * t + ii], xil = Xr[l * t + ii];
+                for (int k = 0; k < KB; ++k) {
+                    xa[k] = *reinterpret_cast<const double2 *>(xrow + 8 * k);
+                    const double2 a21 = *reinterpret_cast<const double2 *>(s21 + 8 * k);
+                    const double2 a11 = *reinterpret_cast<const double2 *>(s11 + 8 * k);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const double xlj = Xc[l * t + jq + k];
-                        t1[k] = fma(a21, xlj, t1[k]);
-                        t2[k] = fma(xil, S12c[l * t + jq + k], t2[k]);
-                        st[k] = fma(a11, xlj, st[k]);
+                    for (int u = 0; u < CPW; ++u) {
+                        if (wj + u >= MT) break;
+                        const int o = (8 * (wj + u) + fr) * LD + 8 * k + 2 * fq;
+                        const double2 xb = *reinterpret_cast<const double2 *>(Xc + o);
+                        const double2 b12 = *reinterpret_cast<const double2 *>(S12c + o);
+                        dmma(st[u][0], st[u][1], a11.x, xb.x);
+                        dmma(t1[u][0], t1[u][1], a21.x, xb.x);
+                        dmma(t2[u][0], t2[u][1], xa[k].x, b12.x);
+                        dmma(st[u][0], st[u][1], a11.y, xb.y);
+                        dmma(t1[u][0], t1[u][1], a21.y, xb.y);
+                        dmma(t2[u][0], t2[u][1], xa[k].y, b12.y);
                     }
                 }
-            // (rows ii >= t are not in the tile: their slots belong to the next column)
-            if (ii < t) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (jq + k < t) STt[(jq + k) * t + ii] = st[k];
-            }
-            cl.sync();  // every tile's st1 = s11 sa0 is in place
-            for (int g = 0; g < kLagTileGrid; ++g) {
-                const double *stt = cl.map_shared_rank(STt, g * kLagTileGrid + q);
-                for (int e = tid; e < t * t; e += kLagThreads) {
-                    const int c = e / t, r = e % t;
-                    const int lc = g * t + r;
-                    if (lc < m) STc[lc * t + c] = stt[e];
+                for (int u = 0; u < CPW; ++u) {
+                    if (wj + u >= MT) break;
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        part[u][e] = t2[u][e] + (t1[u][e] + c22[u][e]);
+                        const int o = (8 * (wj + u) + 2 * fq + e) * LD + i0 + i;
+#pragma unroll
+                        for (int g = 0; g < G; ++g) st_to[g][o] = st[u][e];
+                    }
                 }
             }
-            __syncthreads();
-            // sa1 += sa0 st1 (cpsd.c:463-468); st1 = sa1 - sa0 (:469-470)
-            double s2[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) s2[k] = 0.0;
-            if (rowok)
-                for (int l = 0; l < m; ++l) {
-                    const double xil = Xr[l * t + ii];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) s2[k] = fma(xil, STc[l * t + jq + k], s2[k]);
-                }
+            cl.sync();  // every st1 = s11 sa0 has arrived; nobody reads Xr or Xc any more
             double bestv = -1.0;
-            long besti = 0x7fffffff;
-            double *nxt = Xt + (half ^ 1) * t * t;
+            int besti = 0x7fffffff;
+            if (wact) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int jj = jq + k;
-                if (rowok && jj < nc) {
-                    // sa1 = s22, += s21 sa0, += sa0 s12, += sa0 st1: the
-                    // order of lagrange_kernel
-                    const double sa1 = s2[k] + (t2[k] + (t1[k] + S22t[jj * t + ii]));
-                    const long f = (i0 + ii) + (long)(j0 + jj) * m;
-                    nxt[jj * t + ii] = sa1;
-                    a.X1[f] = sa1;
-                    const double d = sa1 - Xt[half * t * t + jj * t + ii];
-                    a.st1[f] = d;
-                    const double ad = fabs(d);
-                    if (ad > bestv || (ad == bestv && f < besti)) {
-                        bestv = ad;
-                        besti = f;
+                for (int u = 0; u < CPW; ++u) {
+                    if (wj + u >= MT) break;
+                    double t4[2] = {0.0, 0.0};
+#pragma unroll
+                    for (int k = 0; k < KB; ++k) {
+                        const double2 sb =
+                            *reinterpret_cast<const double2 *>(STc + (8 * (wj + u) + fr) * LD + 8 * k + 2 * fq);
+                        dmma(t4[0], t4[1], xa[k].x, sb.x);
+                        dmma(t4[0], t4[1], xa[k].y, sb.y);
                     }
+                    const int jl = 8 * (wj + u) + 2 * fq;
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        // sa1 = s22, += s21 sa0, += sa0 s12, += sa0 st1 (cpsd.c:463-470)
+                        const double v = t4[e] + part[u][e];
+                        const int ri = i0 + i, cj = j0 + jl + e;
+                        if (ri < m && cj < m) {
+                            const double d = v - x[u][e], ad = fabs(d);
+                            const int f = ri + cj * m;
+                            a.st1[f] = d;
+                            if (f == 0) a.X1[0] = v;
+                            if (ad > bestv || (ad == bestv && f < besti)) {
+                                bestv = ad;
+                                besti = f;
+                            }
+                        }
+                        x[u][e] = v;
+#pragma unroll
+                        for (int g = 0; g < G; ++g) xc_to[g][(jl + e) * LD + i0 + i] = v;
+                    }
+#pragma unroll
+                    for (int g = 0; g < G; ++g)
+                        *reinterpret_cast<double2 *>(xr_to[g] + i * LD + j0 + jl) = make_double2(x[u][0], x[u][1]);
                 }
             }
             // tile argmax (first column-major index of the largest |st1|, as idamax)
-            __shared__ double shv[kLagThreads / 32];
-            __shared__ long shi[kLagThreads / 32];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const double ov = __shfl_xor_sync(0xffffffffu, bestv, o);
-                const long oi = __shfl_xor_sync(0xffffffffu, besti, o);
-                if (ov > bestv || (ov == bestv && oi < besti)) {
-                    bestv = ov;
-                    besti = oi;
-                }
-            }
-            if ((tid & 31) == 0) {
-                shv[tid >> 5] = bestv;
-                shi[tid >> 5] = besti;
+            unsigned hi, lo;
+            int at;
+            warp_argmax(bestv, besti, hi, lo, at);
+            if (lane == 0) {
+                wslot[warp][0] = hi;
+                wslot[warp][1] = lo;
+                wslot[warp][2] = (unsigned)at;
             }
             __syncthreads();
-            if (tid == 0) {
-                for (int w = 1; w < kLagThreads / 32; ++w)
-                    if (shv[w] > bestv || (shv[w] == bestv && shi[w] < besti)) {
-                        bestv = shv[w];
-                        besti = shi[w];
-                    }
-                slot[2 * rank] = bestv;
-                slot[2 * rank + 1] = (double)besti;
-            }
-            cl.sync();  // every tile's candidate, st1 and sa1 are in place
-            double gv = -1.0;
-            long gi = 0x7fffffff;
-            for (int r = 0; r < kLagTileGrid * kLagTileGrid; ++r) {
-                const double *sl = cl.map_shared_rank(slot, r);
-                const double v = sl[0];
-                const long ix = (long)sl[1];
-                if (v > gv || (v == gv && ix < gi)) {
-                    gv = v;
-                    gi = ix;
+            if (warp == 0) {
+                constexpr int NW = kLagThreads / 32;
+                combine_argmax(lane < NW ? wslot[lane][0] : 0u, lane < NW ? wslot[lane][1] : 0u,
+                               lane < NW ? wslot[lane][2] : 0x7fffffffu, hi, lo, at);
+                if (lane < G * G) {  // to every CTA
+                    unsigned *to = cl.map_shared_rank(&slot[0][0], lane) + 4 * rank;
+                    to[0] = hi;
+                    to[1] = lo;
+                    to[2] = (unsigned)at;
                 }
             }
+            cl.sync();  // every candidate, difference and new sa0 is in place
+            combine_argmax(lane < G * G ? slot[lane][0] : 0u, lane < G * G ? slot[lane][1] : 0u,
+                           lane < G * G ? slot[lane][2] : 0x7fffffffu, hi, lo, at);
             // idamax returns an index in 1..kk even when every entry is NaN
-            if (gi < 0 || gi >= kk) gi = 0;
+            if (at < 0 || at >= kk) at = 0;
             // the reference reads st1 at idamax's 1-based result (cpsd.c:471):
             // the element after the largest; past the end of st1 lies sa1
-            const long nx = gi + 1;
-            const double adiff = fabs(nx < ne02 ? a.st1[nx] : a.X1[nx - ne02]);
+            const long nx = (long)at + 1;
+            const double adiff = fabs(__ldcg(nx < ne02 ? a.st1 + nx : a.X1 + (nx - ne02)));
             done = adiff < 1e-15;
-            half ^= 1;  // sa1 becomes sa0 (when done, it is the result)
+            // the candidates and differences are written again only after the
+            // next iteration's first barrier
         }
         if (!done && rank == 0 && tid == 0) atomicAdd(a.fail, 1);
         // lmd = the last sa1 (cpsd.c:478)
-        const double *fin = Xt + half * t * t;
-        for (int e = tid; e < t * t; e += kLagThreads) {
-            const int jj = e / t, r = e % t;
-            if (r < nr && jj < nc) a.lmd[ms * ne02 + (i0 + r) + (long)(j0 + jj) * m] = fin[e];
-        }
-        cl.sync();  // the slots and tiles are reused by the next spin
+        if (wact)
+#pragma unroll
+            for (int u = 0; u < CPW; ++u)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int ri = i0 + i, cj = j0 + 8 * (wj + u) + 2 * fq + e;
+                    if (wj + u < MT && ri < m && cj < m) a.lmd[ms * ne02 + ri + (long)cj * m] = x[u][e];
+                }
+        cl.sync();  // the panels and slots are reused by the next spin; no CTA leaves before its peers' stores
     }
 }
 

@@ -61,18 +61,6 @@ size_t small_smem_bytes(int ne0)
     return sizeof(double) * (red > solve ? red : solve);
 }
 
-// largest |d| over a warp with the smallest index among equals, as idamax
-// (NaN never wins; -1 where every entry was NaN); all lanes get the result
-CPSD_D void warp_argmax(double ad, int idx, unsigned &hi, unsigned &lo, int &at)
-{
-    const bool ok = ad >= 0.0;  // false for NaN and for "no entry" (-1)
-    const unsigned long long k = ok ? (unsigned long long)__double_as_longlong(ad) : 0ull;
-    const unsigned h = (unsigned)(k >> 32), l = (unsigned)k;
-    hi = __reduce_max_sync(0xffffffffu, h);
-    lo = __reduce_max_sync(0xffffffffu, h == hi ? l : 0u);
-    at = (int)__reduce_min_sync(0xffffffffu, (ok && h == hi && l == lo) ? (unsigned)idx : 0x7fffffffu);
-}
-
 // cpsd.c:439-478 on the summed overlaps S (tiles in the order they were
 // accumulated).  Tile (I, J) of X belongs to one warp.  A fragment of the
 // product register layout (row lane / 4, columns 2 (lane % 4) + e) is an A
@@ -215,11 +203,8 @@ CPSD_D void small_lagrange(const LagArgs &a, int ms, int m, const double *S, dou
         }
         sync();
         if constexpr (MT > 1) {  // every warp combines the warps' candidates and takes the same decision
-            const unsigned h = lane < kSmWarps ? slot[lane][0] : 0u, l = lane < kSmWarps ? slot[lane][1] : 0u;
-            const unsigned s = lane < kSmWarps ? slot[lane][2] : 0x7fffffffu;
-            hi = __reduce_max_sync(0xffffffffu, h);
-            lo = __reduce_max_sync(0xffffffffu, h == hi ? l : 0u);
-            at = (int)__reduce_min_sync(0xffffffffu, (h == hi && l == lo) ? s : 0x7fffffffu);
+            combine_argmax(lane < kSmWarps ? slot[lane][0] : 0u, lane < kSmWarps ? slot[lane][1] : 0u,
+                           lane < kSmWarps ? slot[lane][2] : 0x7fffffffu, hi, lo, at);
         }
         // idamax returns an index in 1..kk even when every entry is NaN: the
         // sentinel must never reach the read below
