@@ -434,9 +434,9 @@ void cpsd_gpu_batch_destroy(cpsd_gpu_batch *b);
  * builds s22, s21, s12 and s11 from such products, one pair at a time.
  * method: CPSD_GEMM_FP64 or CPSD_GEMM_TF32X3.  Runs on `stream` (NULL: the
  * legacy stream) of the current device and returns after it finishes; the
- * split-K workspace comes from a memory pool the library keeps per device (at
- * most 64 MiB while idle; calls on several threads or streams get their own;
- * the pool does not survive a cudaDeviceReset).
+ * split-K workspace is an 8 MiB device array of the library, held by one call
+ * at a time, or comes from a memory pool it keeps per device (at most 64 MiB
+ * while idle; neither survives a cudaDeviceReset).
  */
 int cpsd_overlap_tn(int method, int M, int N, int K, const double *A, long lda, const double *B, long ldb,
                     const double *w, double *C, long ldc, void *stream);

@@ -3837,6 +3837,11 @@ void cpsd_gpu_destroy(cpsd_gpu_ctx *c)
 constexpr size_t kNoAllocHeadDoubles = 32;
 constexpr size_t kNoAllocScratchDoubles = kNoAllocHeadDoubles + CPSD_NOALLOC_MAX_DOUBLES;  // 8 MiB
 static __device__ __align__(256) double g_overlap_scratch[kNoAllocScratchDoubles];
+// The same for cpsd_overlap_tn, held by one call at a time (its calls wait for
+// their work, so the lock covers the use): a call that finds it taken, or
+// needs more, takes its workspace from the pool.  The timeout word stays zero
+// between calls.
+static __device__ __align__(256) double g_overlap_workspace[kNoAllocScratchDoubles];
 
 namespace {
 
@@ -3864,19 +3869,21 @@ int noalloc_scratch(double **out)
     return CPSD_OK;
 }
 
-// Workspaces of cpsd_overlap_tn: a memory pool of this library's own per
-// device, so that a call's stream-ordered allocation is served from what
-// earlier calls freed (cudaMalloc and cudaFree took 0.6 ms of a 0.75 ms call
-// at 128 x 128 x 38138).  The pool keeps at most kOverlapPoolKeep bytes when
-// idle; more goes back to the device at the call's synchronisation.  Calls on
-// several threads or streams get workspaces of their own.
+// Workspaces of cpsd_overlap_tn beyond g_overlap_workspace: a memory pool of
+// this library's own per device, so that a call's stream-ordered allocation is
+// served from what earlier calls freed.  (cudaMalloc and cudaFree took 0.6 ms of
+// a 0.75 ms call at 128 x 128 x 38138; the pool's calls take 8 us, which the
+// smallest products of 40 us notice: hence the array before it.)  The pool keeps
+// at most kOverlapPoolKeep bytes when idle; more goes back to the device at the
+// call's synchronisation.  Calls on several threads or streams get workspaces
+// of their own.
 constexpr size_t kOverlapPoolKeep = (size_t)64 << 20;
 cudaMemPool_t g_overlap_pool[kNoAllocMaxDevices] = {};
+double *g_overlap_ws[kNoAllocMaxDevices] = {};
+std::mutex g_overlap_mu[kNoAllocMaxDevices];
 
-int overlap_pool(cudaMemPool_t *out)
+int overlap_pool(int dev, cudaMemPool_t *out)
 {
-    int dev = 0;
-    CK(cudaGetDevice(&dev));
     if (dev < 0 || dev >= kNoAllocMaxDevices) return CPSD_ERR_ARG;
     std::lock_guard<std::mutex> lock(g_noalloc_mu);
     if (!g_overlap_pool[dev]) {
@@ -3889,7 +3896,8 @@ int overlap_pool(cudaMemPool_t *out)
         cudaMemPool_t p = nullptr;
         CK(cudaMemPoolCreate(&p, &pr));
         uint64_t keep = kOverlapPoolKeep;
-        const cudaError_t e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+        cudaError_t e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e == cudaSuccess) e = cudaGetSymbolAddress((void **)&g_overlap_ws[dev], g_overlap_workspace);
         if (e != cudaSuccess) cudaMemPoolDestroy(p);
         CK(e);
         g_overlap_pool[dev] = p;
@@ -3911,12 +3919,25 @@ int cpsd_overlap_tn(int method, int M, int N, int K, const double *A, long lda, 
     if (!A || !B || !C) return CPSD_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     const bool tc = method != CPSD_GEMM_FP64;
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
     cudaMemPool_t pool = nullptr;
-    int rc = overlap_pool(&pool);
+    int rc = overlap_pool(dev, &pool);
     if (rc) return rc;
     const size_t cap = std::max<size_t>((size_t)M * N, (size_t)4 << 20);
-    const TnPlan pl = tn_plan(M, N, K, 1, tc, cap, device_sms());
+    // the array holds every product but the largest, with fewer splits where
+    // the plan's would not fit and it still fills the SMs twice
+    TnPlan pl = tn_plan(M, N, K, 1, tc, cap, device_sms());
+    size_t ws_cap = cap;
+    if ((size_t)pl.splits * M * N > (size_t)CPSD_NOALLOC_MAX_DOUBLES) {
+        const TnPlan small = tn_plan(M, N, K, 1, tc, (size_t)CPSD_NOALLOC_MAX_DOUBLES, device_sms());
+        if (2 * small.splits >= pl.splits && (size_t)small.splits * M * N <= (size_t)CPSD_NOALLOC_MAX_DOUBLES) {
+            pl = small;
+            ws_cap = (size_t)CPSD_NOALLOC_MAX_DOUBLES;
+        }
+    }
     // the timeout word of the tensor-core pipeline, then the partials
+    std::unique_lock<std::mutex> held(g_overlap_mu[dev], std::defer_lock);
     struct Scratch {
         cudaStream_t s;
         double *p = nullptr;
@@ -3925,16 +3946,26 @@ int cpsd_overlap_tn(int method, int M, int N, int K, const double *A, long lda, 
             if (p) cudaFreeAsync(p, s);
         }
     } sc{s};
-    CK(cudaMallocFromPoolAsync((void **)&sc.p, sizeof(double) * (kNoAllocHeadDoubles + (size_t)pl.splits * M * N), pool, s));
-    int *err = reinterpret_cast<int *>(sc.p);
-    if (tc) CK(cudaMemsetAsync(err, 0, sizeof(int), s));
-    (void)launch_tn(M, N, K, 1, &A, lda, &B, ldb, w, 1.0, 0.0, &C, ldc, tc, sc.p + kNoAllocHeadDoubles, cap, err, s);
+    double *ws = nullptr;
+    if ((size_t)pl.splits * M * N <= (size_t)CPSD_NOALLOC_MAX_DOUBLES && held.try_lock()) {
+        ws = g_overlap_ws[dev];
+    } else {
+        CK(cudaMallocFromPoolAsync((void **)&sc.p, sizeof(double) * (kNoAllocHeadDoubles + (size_t)pl.splits * M * N),
+                                   pool, s));
+        ws = sc.p;
+    }
+    int *err = reinterpret_cast<int *>(ws);
+    if (tc && sc.p) CK(cudaMemsetAsync(err, 0, sizeof(int), s));
+    (void)launch_tn(M, N, K, 1, &A, lda, &B, ldb, w, 1.0, 0.0, &C, ldc, tc, ws + kNoAllocHeadDoubles, ws_cap, err, s);
     CK(cudaGetLastError());
     int herr = 0;
     if (tc) CK(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CK(cudaFreeAsync(sc.p, s));
-    sc.p = nullptr;
+    if (sc.p) {
+        CK(cudaFreeAsync(sc.p, s));
+        sc.p = nullptr;
+    }
     CK(cudaStreamSynchronize(s));
+    if (herr && held.owns_lock()) CK(cudaMemset(err, 0, sizeof(int)));
     return herr ? CPSD_ERR_TIMEOUT : CPSD_OK;
 }
 
