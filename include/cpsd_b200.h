@@ -107,7 +107,9 @@ enum { CPSD_PREC_FP64 = 0, CPSD_PREC_MIXED = 1 };
  * memory, FP64 split-K sums), about FP32 accuracy.  CPSD_GEMM_TF32X3 moves
  * the KB projector contraction and back-projection (and the learned step's
  * residual) to the tensor cores; CPSD_GEMM_TF32X3_OVERLAPS moves the three
- * Lagrange overlaps and the constraint correction as well.  The
+ * Lagrange overlaps and the constraint correction as well (products of at most
+ * 64 x 64 outputs, and all of a cell of at most 32 bands per spin, stay FP64:
+ * faster there).  The
  * Lagrange solve divides (1 - <c2|c2>) by dte (about 1e-2), so FP32-level
  * overlaps cost about 1e-6 relative in the energy per step: follow such a
  * run with FP64 steps. */
@@ -299,7 +301,8 @@ int cpsd_gpu_bp_finish(cpsd_gpu_ctx *c, int inner, double *E, double *deltae, do
 typedef struct {
     int plane_occupancy[4]; /* per plane pass (0 density, 1 V psi, 2 potential to r,
                                3 density to G): 0 = the build for one CTA per SM (up to
-                               255 registers a thread), 1 = the one for two (128) */
+                               255 registers a thread, or more threads), 1 = the one for
+                               two (128).  0 and 1 have one build for both choices */
     int tn_ctas_per_sm;     /* split-K target of the weighted TN products: CTAs per SM, 1..8 */
     int density_chunks;     /* band chunks per spin of the density pass */
     int lagrange_solver;    /* more than 32 bands: 1 = 4 x 4 tiled cluster, 2 = column

@@ -976,7 +976,7 @@ const double *Mblk(cpsd_gpu_ctx *c, int ms, int which)
 
 // Cells of at most 32 bands per spin take the 8 x 8 tile kernels of small.cuh
 // for their band-by-band products, in every GEMM mode: at 16 bands (64^3) the
-// three overlaps and the solver take 7 us there against 29 us as 64 x 64 tiles
+// three overlaps and the solver take 16 us there against 33 us as 64 x 64 tiles
 // (FP64, or 3xTF32 on 128 x 128 ones), a reduction and a solver launch.
 bool small_cell(const cpsd_gpu_ctx *c) { return c->ne0 <= kLagSmallMax; }
 
